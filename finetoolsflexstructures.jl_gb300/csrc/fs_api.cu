@@ -53,8 +53,9 @@ int read_status(fs_ctx *c, int *bits)
 
 static void free_pattern(PatternDev &P)
 {
-    dfree(&P.nbr_off); dfree(&P.nbr); dfree(&P.pair_slots); dfree(&P.colpos); dfree(&P.colsrc); dfree(&P.rowlen);
-    dfree(&P.sl_off); dfree(&P.sl_ent); dfree(&P.sl_mir); dfree(&P.lc);
+    dfree(&P.nbr_off); dfree(&P.nbr); dfree(&P.colpos); dfree(&P.colsrc); dfree(&P.rowlen);
+    dfree(&P.sl_off); dfree(&P.sl_last); dfree(&P.src); dfree(&P.item_off); dfree(&P.items);
+    dfree(&P.rowstart);
     dfree(&P.rowptr); dfree(&P.colidx); dfree(&P.diag_rowptr); dfree(&P.diag_colidx);
     dfree(&P.tmp_cnt); dfree(&P.tmp_owner);
     P = PatternDev();
@@ -66,7 +67,6 @@ static void reset_pattern(PatternDev &P)
 {
     P.n = -1;
     P.nnz = 0;
-    P.maxlen = 0;
 }
 
 static void free_mesh(MeshDev &m)
@@ -731,6 +731,8 @@ int fs_element_matrices(fs_ctx *c, int precision, double *out)
     std::vector<int32_t> eor((size_t)m.nelem);
     if (m.nelem)
         FS_CUDA(c, cudaMemcpy(eor.data(), m.elem_of_rank, sizeof(int32_t) * m.nelem, cudaMemcpyDeviceToHost));
+    std::vector<int32_t> cn((size_t)(m.nelem * nen));
+    if (m.nelem) FS_CUDA(c, cudaMemcpy(cn.data(), m.conn, sizeof(int32_t) * cn.size(), cudaMemcpyDeviceToHost));
     std::vector<double> kd;
     std::vector<float> kf;
     if (precision == FS_FP64) {
@@ -748,10 +750,11 @@ int fs_element_matrices(fs_ctx *c, int precision, double *out)
             for (int b = 0; b < nen; b++)
                 for (int i = 0; i < 6; i++)
                     for (int j = 0; j < 6; j++) {
-                        size_t src = stored * r +
-                                     (a <= b ? (size_t)ub(a, b, nen) * 36 + i * 6 + j : (size_t)ub(b, a, nen) * 36 + j * 6 + i);
+                        const size_t src = stored * r + stored_entry(a, b, nen, &cn[(size_t)(r * nen)], i, j);
+                        // float pairs: entries 2q, 2q + 1 as hi, hi, lo, lo
+                        const size_t hi = 2 * src - (src & 1);
                         double v = precision == FS_FP64         ? kd[src]
-                                   : precision == FS_MIXED_COMP ? (double)kf[2 * src] + (double)kf[2 * src + 1]
+                                   : precision == FS_MIXED_COMP ? (double)kf[hi] + (double)kf[hi + 2]
                                                                 : (double)kf[src];
                         o[(6 * a + i) + (size_t)nd * (6 * b + j)] = v;
                     }

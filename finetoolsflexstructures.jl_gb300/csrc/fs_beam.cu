@@ -82,6 +82,16 @@ __global__ void __launch_bounds__(128) k_beam_elements(const MeshDev m, const Be
         for (int bb = a; bb < 2; bb++) {
             double acc[6][6];
             beam_block<WHICH>(e, a, bb, acc);
+            if (a != bb && m.conn[2 * r] > m.conn[2 * r + 1]) {  // the lower node's dofs as rows
+#pragma unroll
+                for (int i = 0; i < 6; i++)
+#pragma unroll
+                    for (int j = 0; j < i; j++) {
+                        const double t = acc[i][j];
+                        acc[i][j] = acc[j][i];
+                        acc[j][i] = t;
+                    }
+            }
             store_block_d(out + ub(a, bb, 2) * 36, acc);
         }
 }
@@ -335,8 +345,9 @@ int fs_beam_element_matrices(fs_ctx *c, int which, int mass_type, double *out)
     FS_TRY(launch_beam_elements(c, which, mass_type));
     const int64_t ne = c->mesh.nelem;
     std::vector<double> blk((size_t)(108 * ne));
-    std::vector<int32_t> eor((size_t)ne);
+    std::vector<int32_t> eor((size_t)ne), cn((size_t)(2 * ne));
     if (ne) {
+        FS_CUDA(c, cudaMemcpyAsync(cn.data(), c->mesh.conn, sizeof(int32_t) * 2 * ne, cudaMemcpyDeviceToHost, c->stream));
         FS_CUDA(c, cudaMemcpyAsync(blk.data(), c->ke, sizeof(double) * 108 * ne, cudaMemcpyDeviceToHost, c->stream));
         FS_CUDA(c, cudaMemcpyAsync(eor.data(), c->mesh.elem_of_rank, sizeof(int32_t) * ne, cudaMemcpyDeviceToHost,
                                    c->stream));
@@ -349,8 +360,7 @@ int fs_beam_element_matrices(fs_ctx *c, int which, int mass_type, double *out)
             for (int b = 0; b < 2; b++)
                 for (int i = 0; i < 6; i++)
                     for (int j = 0; j < 6; j++)
-                        o[(6 * a + i) + 12 * (6 * b + j)] =
-                            a <= b ? k[ub(a, b, 2) * 36 + i * 6 + j] : k[ub(b, a, 2) * 36 + j * 6 + i];
+                        o[(6 * a + i) + 12 * (6 * b + j)] = k[stored_entry(a, b, 2, &cn[(size_t)(2 * r)], i, j)];
     }
     return FS_OK;
 }

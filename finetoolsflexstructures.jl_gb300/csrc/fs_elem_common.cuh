@@ -107,7 +107,8 @@ template <class R, bool PAIR, int NI = 6> struct BlockAcc {
 // sums, entries (i, 2q) and (i, 2q + 1) in one packed register pair.  A row
 // reaching only one entry of a pair adds a zero product to the other, which
 // leaves its sums unchanged; DIAG: only the pairs holding an entry j >= i.
-// store() writes s + (c + d) as (hi, lo) float pairs: c + d rounded (below
+// store() writes s + (c + d) as (hi, lo) float pairs (entries 2q, 2q + 1 as hi,
+// hi, lo, lo: the gather's packed pairs): c + d rounded (below
 // the pair's last bit), then Fast2Sum; DIAG mirrors the entries j < i.
 // LEVELS 2: Dot2 on entry pairs (s, c; what is lost is c's rounding, about
 // 2^-48 of the summed terms per term summed), for elements with few rows per
@@ -169,7 +170,7 @@ template <int NI, int LEVELS = 3> struct PairAcc {
         for (int i = 0; i < NI; i++)
 #pragma unroll
             for (int q = 0; q < 3; q++)
-                o4[3 * i + q] = make_float4(h[i][2 * q], l[i][2 * q], h[i][2 * q + 1], l[i][2 * q + 1]);
+                o4[3 * i + q] = make_float4(h[i][2 * q], h[i][2 * q + 1], l[i][2 * q], l[i][2 * q + 1]);
     }
 };
 template <int NI> struct BlockAcc<float, true, NI> : PairAcc<NI, Q4_PAIR_LEVELS> {};
@@ -247,15 +248,32 @@ __device__ __forceinline__ void gram_rows_h(Acc &acc, const R *base, int r0, int
 template <class R, bool PAIR> struct T3Acc { typedef BlockAcc<R, PAIR> type; };
 template <> struct T3Acc<float, true> { typedef PairAcc<6, T3_PAIR_LEVELS> type; };
 
+// Which off-diagonal blocks (a, b), b > a, of an NN-node element are stored as
+// K_ba, the lower node's dofs being the rows of a stored block: bit NN a + b.
+template <int NN> __device__ __forceinline__ unsigned swapped_blocks(const int32_t *node)
+{
+    unsigned m = 0;
+#pragma unroll
+    for (int a = 0; a < NN; a++)
+#pragma unroll
+        for (int b = a + 1; b < NN; b++) m |= node[a] > node[b] ? 1u << (NN * a + b) : 0u;
+    return m;
+}
+
 // The upper node blocks of an NN-node element: diag(a) computes block
-// (a, a) (its upper triangle), off(a, b) block (a, b) for b > a.
+// (a, a) (its upper triangle), off(p, q, o) block (p, q) into position o, where
+// {p, q} = {a, b}, a < b, ordered as swapped_blocks tells.
 // Plain stores (float or double): one loop over the blocks, not unrolled,
 // choosing the diagonal or the off-diagonal form (the shorter code measured
 // 28 % faster for the float T3 kernel).  Float-pair stores: the diagonal
 // blocks, then the off-diagonal ones (4 % faster for those).
 template <int NN, bool PAIR, class D, class O>
-__device__ __forceinline__ void for_upper_blocks(D diag, O off)
+__device__ __forceinline__ void for_upper_blocks(unsigned swapped, D diag, O off_pq)
 {
+    auto off = [&](int a, int b) {
+        const bool sw = (swapped >> (NN * a + b)) & 1u;
+        off_pq(sw ? b : a, sw ? a : b, ub(a, b, NN));
+    };
     if constexpr (PAIR) {
 #pragma unroll 1
         for (int a = 0; a < NN; a++) diag(a);
@@ -280,12 +298,12 @@ __device__ __forceinline__ void for_upper_blocks(D diag, O off)
 // CompactRows<NN, NS> layout: the products and their order are those of the
 // SPARSE path of write_blocks, so the blocks are bitwise the same.
 template <class R, class S, int NN, int NS>
-__device__ __forceinline__ void write_blocks_compact(const R *rows, S *out)
+__device__ __forceinline__ void write_blocks_compact(const R *rows, unsigned swapped, S *out)
 {
     typedef CompactRows<NN, NS> L;
     constexpr bool PAIR = sizeof(S) == 8 && sizeof(R) == 4;
     for_upper_blocks<NN, PAIR>(
-        [&](int a) {
+        swapped, [&](int a) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
             gram_rows_c<0, 3, 0, 3, L::MS, 3, 0, true, PAIR>(acc, rows, 0, 3, a, a);
@@ -293,12 +311,12 @@ __device__ __forceinline__ void write_blocks_compact(const R *rows, S *out)
             gram_rows_c<3, 6, 3, 6, 3, 0, 3, true, PAIR>(acc, rows + L::DR + 3 * a, 0, 1, a, a);
             acc.template store<true>(out + ub(a, a, NN) * 36);
         },
-        [&](int a, int b) {
+        [&](int a, int b, int o) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
             gram_rows_c<0, 3, 0, 3, L::MS, 3, 0, false, PAIR>(acc, rows, 0, 3, a, b);
             gram_rows_c<0, 6, 0, 6, L::BSS, 6, 0, false, PAIR>(acc, rows + L::BS, 0, 3 + NS, a, b);
-            acc.store(out + ub(a, b, NN) * 36);
+            acc.store(out + o * 36);
         });
 }
 
@@ -309,12 +327,12 @@ __device__ __forceinline__ void write_blocks_compact(const R *rows, S *out)
 // rotations of one node each); their structurally zero products are
 // skipped, in the same row order, so the sums are those of the dense loop.
 template <class R, class S, int NN, bool SPARSE>
-__device__ __forceinline__ void write_blocks(const R *rows, int nrows, S *out)
+__device__ __forceinline__ void write_blocks(const R *rows, int nrows, unsigned swapped, S *out)
 {
     constexpr bool PAIR = sizeof(S) == 8 && sizeof(R) == 4;
     const int ND = 6 * NN;
     for_upper_blocks<NN, PAIR>(
-        [&](int a) {
+        swapped, [&](int a) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
             if (SPARSE) {
@@ -326,7 +344,7 @@ __device__ __forceinline__ void write_blocks(const R *rows, int nrows, S *out)
             }
             acc.template store<true>(out + ub(a, a, NN) * 36);
         },
-        [&](int a, int b) {
+        [&](int a, int b, int o) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
             if (SPARSE) {
@@ -335,7 +353,7 @@ __device__ __forceinline__ void write_blocks(const R *rows, int nrows, S *out)
             } else {
                 gram_rows<0, 6, 0, 6, false, PAIR>(acc, rows, ND, 0, nrows, a, b);
             }
-            acc.store(out + ub(a, b, NN) * 36);
+            acc.store(out + o * 36);
         });
 }
 

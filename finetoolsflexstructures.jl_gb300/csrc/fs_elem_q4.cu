@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const M
     __syncwarp();
     if (!active) return;
     S *out = ke + r * (10 * 36);
+    const unsigned swapped = swapped_blocks<4>(m.conn + r * 4);
     constexpr bool PAIR = sizeof(S) == 8 && sizeof(R) == 4;
     // The element's ten upper node blocks over its four lanes, every lane
     // running the same code at each step: first the diagonal block (qp, qp)
@@ -215,9 +216,12 @@ __global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const M
 #pragma unroll 1
     for (int t = 0; t < 3; t++) {
         const int u = qp + 4 * t, ob = u < 6 ? u : u - 6, i0 = u < 6 ? 0 : 3;
-        // off-diagonal block ob: (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
-        const int a = ob < 3 ? 0 : (ob < 5 ? 1 : 2);
-        const int b = ob < 3 ? ob + 1 : (ob < 5 ? ob - 1 : 3);
+        // off-diagonal block ob: (0,1) (0,2) (0,3) (1,2) (1,3) (2,3), the lower
+        // node's dofs as its rows
+        const int a0 = ob < 3 ? 0 : (ob < 5 ? 1 : 2);
+        const int b0 = ob < 3 ? ob + 1 : (ob < 5 ? ob - 1 : 3);
+        const bool sw = (swapped >> (4 * a0 + b0)) & 1u;
+        const int a = sw ? b0 : a0, b = sw ? a0 : b0;
         BlockAcc<R, PAIR, 3> acc;
         acc.zero();
         if constexpr (!COMP) {
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const M
         } else {
             gram_rows_h<0, 6, ND, 6>(acc, rows, 0, 36, a, b, i0);
         }
-        acc.store(out + ub(a, b, 4) * 36 + 6 * i0);
+        acc.store(out + ub(a0, b0, 4) * 36 + 6 * i0);
     }
 }
 

@@ -38,10 +38,11 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     const GroupConst *gc = COMP ? &m.groups[in.group] : nullptr;
     int st = t3_rows<R, COMP, AVGK, !COMP>(in, mc, gc, rows, ND);
     if (st) atomicOr(status, DEV_NEG_DRILL);
+    const unsigned swapped = swapped_blocks<3>(m.conn + r * 3);
     if constexpr (COMP)
-        write_blocks<R, S, 3, false>(rows, NR, ke + r * (6 * 36));
+        write_blocks<R, S, 3, false>(rows, NR, swapped, ke + r * (6 * 36));
     else
-        write_blocks_compact<R, S, 3, NS>(rows, ke + r * (6 * 36));
+        write_blocks_compact<R, S, 3, NS>(rows, swapped, ke + r * (6 * 36));
 }
 
 template <class R, bool COMP, bool AVGK, class S = R>

@@ -33,9 +33,19 @@ enum : int {
 static const int MAX_PAIRS_PER_NODE = 64;   // elements meeting at one node
 
 // Element matrices are stored as their upper 6x6 node blocks (a <= b) only,
-// row-major inside a block; ub(a, b) is the block's position.
+// row-major inside a block; ub(a, b) is the block's position.  A block's rows
+// are the dofs of the lower of the two (global) nodes: at ub(a, b) lies K_ab,
+// or K_ba when node a is above node b.
 __host__ __device__ __forceinline__ int n_upper_blocks(int nen) { return nen * (nen + 1) / 2; }
 __host__ __device__ __forceinline__ int ub(int a, int b, int nen) { return a * nen - a * (a - 1) / 2 + (b - a); }
+// where entry (i, j) of node block (a, b) of an element with the (global)
+// nodes `node` is stored, in entries from the element's first
+__host__ __device__ __forceinline__ int stored_entry(int a, int b, int nen, const int32_t *node, int i, int j)
+{
+    const bool rows_a = node[a] < node[b] || (node[a] == node[b] && a <= b);  // stored with node a's dofs as rows
+    return (a <= b ? ub(a, b, nen) : ub(b, a, nen)) * 36 + (rows_a ? 6 * i + j : 6 * j + i);
+}
+static const int GATHER_GROUP = 64;         // nodes whose own blocks lie together in the gather's list
 static const int MAX_NBRS = 255;            // neighbour nodes of one node (slots are 8-bit)
 
 struct MeshDev {
@@ -59,30 +69,42 @@ struct MeshDev {
     int32_t *elem_pair = nullptr;  // per rank x nen: pair index
 };
 
+// One block of the assembled matrix for the value gather: the node pair
+// (r, s), r <= s; k, m: the neighbour entries of s in r's list and of r in s's
+// (6 k and 6 m index colpos); cnt element blocks add up to it, in ascending
+// assembly rank: e0, e1 (the first again when there is only one), and src[more
+// + q] for the q-th of them (cnt 0: a node of no element, nothing to write).
+// A contribution is the position of a stored element block (in blocks), with
+// the top bit set when it is read transposed (two nodes of one element that
+// are the same node).  All of these fit 31 or 32 bits for any mesh whose
+// element matrices fit the device's memory.
+struct __align__(32) GatherItem {
+    uint32_t r, s, k, m;
+    uint32_t cnt, e0, e1, more;
+};
+
 struct PatternDev {
     int64_t n = -1;              // matrix size the pattern is built for
     int64_t nnz = 0;
-    int maxlen = 0;              // longest row
     int64_t *nbr_off = nullptr;  // nnodes + 1
     int32_t *nbr = nullptr;      // neighbour nodes, sorted
-    uint32_t *pair_slots = nullptr;  // per pair: 8-bit slot of each element node
     int16_t *colpos = nullptr;   // per node: 6 x nnbr positions in the row (or -1)
     uint16_t *colsrc = nullptr;  // per node: for row position j, neighbour slot * 6 + component
-    // per (node, neighbour slot): the node's contributions to that slot's columns, in
-    // ascending pair order; an entry is q | b << 6 | (b < a_q) << 8 with q the pair
-    // index within the node (< 64), b the element node at that slot, a_q the node's
-    // own element node (the block is the mirror of an upper block when b < a_q).
-    // The entries of node r start at pp[r] * nen; sl_off gives each slot's start.
-    uint16_t *sl_off = nullptr;  // per (node, slot), relative to the node's first entry
-    uint16_t *sl_ent = nullptr;  // npairs * nen
+    // per (node, neighbour slot of the node itself or a higher one): the node's
+    // contributions to that slot's columns, in ascending pair order (GatherItem's
+    // form).  Those of node r start at src[pp[r] * nen]; sl_off gives each slot's
+    // start.
+    uint16_t *sl_off = nullptr;  // per (node, slot), relative to the node's first contribution
+    uint16_t *sl_last = nullptr; // per node: end of its last slot's contributions
+    uint32_t *src = nullptr;     // npairs * nen
     int32_t *rowlen = nullptr;   // per node: row length L
-    // per (node, slot): node-block pairs summed once (k_slot_mirror); sym false
-    // when the neighbour entry indices would not fit 28 bits (every node sums
-    // its own rows)
-    uint32_t *sl_mir = nullptr;
-    int32_t *lc = nullptr;       // per node: row positions summed with pairs summed once (rows <= 64)
-    int maxlc = 0;               // longest of those (the longest row without sym)
-    bool sym = false;
+    // the gather's blocks, by groups of GATHER_GROUP nodes (the nodes' own blocks,
+    // then the off-diagonal ones node by node), and where the rows of each
+    // node's dofs start (-1: not in the matrix)
+    int64_t nitems = 0;
+    int64_t *item_off = nullptr;  // nnodes + 1: blocks of the nodes before
+    GatherItem *items = nullptr;  // null: positions beyond 32 bits
+    int64_t *rowstart = nullptr;  // 6 per node
     int64_t *rowptr = nullptr;   // n + 1
     int32_t *colidx = nullptr;   // nnz, 0-based
     int64_t *diag_rowptr = nullptr;  // diagonal pattern (n + 1)
@@ -90,9 +112,9 @@ struct PatternDev {
     int64_t *tmp_cnt = nullptr;      // temporaries of the symbolic phase
     int32_t *tmp_owner = nullptr;
     // allocated capacities (elements): a rebuild reuses the buffers that fit
-    size_t cap_nbr_off = 0, cap_nbr = 0, cap_pair_slots = 0, cap_colpos = 0, cap_colsrc = 0, cap_rowlen = 0,
-           cap_sl_off = 0, cap_sl_ent = 0, cap_rowptr = 0, cap_colidx = 0, cap_diag_rowptr = 0,
-           cap_diag_colidx = 0, cap_tmp_cnt = 0, cap_tmp_owner = 0, cap_sl_mir = 0, cap_lc = 0;
+    size_t cap_nbr_off = 0, cap_nbr = 0, cap_colpos = 0, cap_colsrc = 0, cap_rowlen = 0, cap_sl_off = 0, cap_sl_last = 0, cap_src = 0,
+           cap_item_off = 0, cap_items = 0, cap_rowstart = 0, cap_rowptr = 0, cap_colidx = 0, cap_diag_rowptr = 0,
+           cap_diag_colidx = 0, cap_tmp_cnt = 0, cap_tmp_owner = 0;
 };
 
 }  // namespace fs
@@ -185,7 +207,7 @@ struct fs_ctx {
     struct Tune {
         int mode = -1;         // -1: not read yet (FLEXSHELL_AUTOTUNE), 0 off, 1 on, 2 re-tune
         int elem_epb = 0;      // elements per block
-        int gather_warps = 0;  // warps (nodes) per block
+        int gather_warps = 0;  // warps per block
         int gather_once = -1;  // node-block pairs summed once: -1 default (yes), 0 no, 1 yes
         bool from_tuner = false;
     } tune;
@@ -256,7 +278,6 @@ int explicit_launch_steps(fs_ctx *c, int64_t nsteps);
 int autotune_shell(fs_ctx *c, int precision);
 size_t t3_smem(int precision, bool avgk, bool layered, int epb);
 size_t entry_bytes(int precision);
-size_t gather_smem_bytes(int precision, int nen, int warps);
 int run_t3_any(fs_ctx *c, int precision, void *ke);
 int run_q4_any(fs_ctx *c, int precision, void *ke);
 size_t q4_smem(int precision, bool layered, int epb);

@@ -10,12 +10,11 @@
 // block (6 of 9 blocks for T3, 10 of 16 for Q4); the gather reads a lower
 // block as the transpose of its mirror.
 //
-// Gather.  One warp owns one node, i.e. the six CSR rows of its dofs.  It
-// walks the node's (element, local node) pairs in ascending assembly rank
-// and adds each slab into a double accumulator, so every CSR value is the
-// left-to-right sum of its element contributions in assembly order, as
-// Julia's sparse(I, J, V) combines duplicates.  No atomics: the result is
-// bitwise reproducible.
+// Gather.  Eighteen threads own one 6x6 block of the assembled matrix and add
+// the element blocks that touch it in ascending assembly rank, so every CSR
+// value is the left-to-right sum of its element contributions in assembly
+// order, as Julia's sparse(I, J, V) combines duplicates.  No atomics: the
+// result is bitwise reproducible.
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -331,8 +330,8 @@ int launch_elements_to(fs_ctx *c, int precision, void *ke)
 // tile-shape autotuner
 // ---------------------------------------------------------------------------
 // Candidates: elements per block of the element kernel (T3: 32, 64, 128;
-// Q4: 8, 16, 32, as far as their shared memory fits in 227 KB) and warps
-// per block of the gather (4, 8, 16).  Each candidate is timed on the
+// Q4: 8, 16, 32, as far as their shared memory fits in 227 KB) and the block
+// size of the gather (4, 8, 16 times 36 threads).  Each candidate is timed on the
 // context's own mesh with CUDA events (best of three launches), the element
 // kernel first, then the gather on its output.  The choice is keyed on
 // element family, precision, the average-K option and log2 of the element
@@ -350,7 +349,7 @@ struct TuneKey {
 };
 std::mutex g_tune_mu;
 struct TuneVal {
-    int epb, warps, once;
+    int epb, warps;
 };
 std::map<TuneKey, TuneVal> g_tune;
 const size_t SMEM_MAX = 227 * 1024;
@@ -400,7 +399,7 @@ int autotune_shell(fs_ctx *c, int precision)
         if (it != g_tune.end()) {
             c->tune.elem_epb = it->second.epb;
             c->tune.gather_warps = it->second.warps;
-            c->tune.gather_once = it->second.once;
+            c->tune.gather_once = 1;
             c->tune.from_tuner = true;
             return FS_OK;
         }
@@ -423,30 +422,24 @@ int autotune_shell(fs_ctx *c, int precision)
     }
     c->tune.elem_epb = best_e;
     FS_TRY(launch_elements(c, precision));  // the gather candidates read these element matrices
-    // gather: warps per block, and whether node-block pairs are summed once
-    // (with transposed copies) or by both nodes; bitwise the same values
-    int best_w = 0, best_o = 1;
+    // gather: the block size
+    int best_w = 0;
     best_ms = 1e30f;
+    c->tune.gather_once = 1;
     for (int w : {4, 8, 16}) {
-        if (gather_smem_bytes(precision, m.nen, w) > SMEM_MAX) continue;
-        for (int once : {1, 0}) {
-            c->tune.gather_warps = w;
-            c->tune.gather_once = once;
-            float ms = 0.f;
-            FS_TRY(time_best(c, run_gather_once, precision, &ms));
-            if (ms < best_ms) {
-                best_ms = ms;
-                best_w = w;
-                best_o = once;
-            }
+        c->tune.gather_warps = w;
+        float ms = 0.f;
+        FS_TRY(time_best(c, run_gather_once, precision, &ms));
+        if (ms < best_ms) {
+            best_ms = ms;
+            best_w = w;
         }
     }
     c->tune.gather_warps = best_w;
-    c->tune.gather_once = best_o;
     c->tune.from_tuner = true;
     if (c->tune.mode == 2) c->tune.mode = 1;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune[key] = {best_e, best_w, best_o};
+    g_tune[key] = {best_e, best_w};
     return FS_OK;
 }
 

@@ -307,7 +307,7 @@ __device__ int node_neighbors(int64_t r, int nen, const int64_t *pp, const int32
 }
 
 __global__ void k_count_nbrs(int64_t nnodes, int nen, const int64_t *pp, const int32_t *pair_e,
-                             const int32_t *conn, int64_t *cnt, int *status)
+                             const int32_t *conn, int64_t *cnt, int64_t *upper, int *status)
 {
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nnodes) return;
@@ -315,13 +315,15 @@ __global__ void k_count_nbrs(int64_t nnodes, int nen, const int64_t *pp, const i
     int n = node_neighbors(r, nen, pp, pair_e, conn, buf);
     if (n > MAX_NBRS) atomicOr(status, DEV_NEIGHBORS);
     cnt[r] = n;
+    int lower = 0;
+    while (lower < n && buf[lower] < r) lower++;
+    upper[r] = max(n - lower, 1);  // r itself and its higher neighbours
 }
 
 __global__ void k_fill_nbrs(int64_t nnodes, int nen, int64_t n_mat, const int64_t *pp,
                             const int32_t *pair_e, const int32_t *conn, const int32_t *dof,
-                            const int64_t *nbr_off, int32_t *nbr, uint32_t *pair_slots,
-                            int16_t *colpos, uint16_t *colsrc, int32_t *rowlen, uint16_t *sl_off,
-                            uint16_t *sl_ent)
+                            const int64_t *nbr_off, int32_t *nbr, int16_t *colpos, uint16_t *colsrc,
+                            int32_t *rowlen, uint16_t *sl_off, uint16_t *last, uint32_t *src)
 {
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nnodes) return;
@@ -330,37 +332,29 @@ __global__ void k_fill_nbrs(int64_t nnodes, int nen, int64_t n_mat, const int64_
     if (n > MAX_NBRS) n = MAX_NBRS;
     int64_t off = nbr_off[r];
     for (int s = 0; s < n; s++) nbr[off + s] = buf[s];
-    // slots of each element node in this node's neighbour list
-    for (int64_t p = pp[r]; p < pp[r + 1]; p++) {
-        int64_t rank = pair_e[p] >> 2;
-        uint32_t packed = 0;
-        for (int k = 0; k < nen; k++) {
-            int32_t v = conn[rank * nen + k];
-            int lo = 0, hi = n - 1;
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                if (buf[mid] < v) lo = mid + 1; else hi = mid;
-            }
-            packed |= (uint32_t)(lo & 0xff) << (8 * k);
-        }
-        pair_slots[p] = packed;
-    }
-    // contribution lists per neighbour slot (ascending pair order)
+    // contribution lists of the node's own and its higher neighbours' slots
+    // (ascending pair order)
     {
         const int64_t p0 = pp[r];
         const int np = (int)min((int64_t)MAX_PAIRS_PER_NODE, pp[r + 1] - p0);
-        uint16_t *ent = sl_ent + p0 * nen;
+        const int nblk = n_upper_blocks(nen);
+        uint32_t *ent = src + p0 * nen;
         int w = 0;
         for (int s = 0; s < n; s++) {
+            const int32_t node = buf[s];
+            if (node < r) continue;
             sl_off[off + s] = (uint16_t)w;
             for (int q = 0; q < np; q++) {
-                const uint32_t packed = pair_slots[p0 + q];
-                const int aq = pair_e[p0 + q] & 3;
+                const int32_t pe = pair_e[p0 + q];
+                const int64_t rank = pe >> 2;
+                const int aq = pe & 3;
                 for (int b = 0; b < nen; b++)
-                    if ((int)((packed >> (8 * b)) & 0xffu) == s)
-                        ent[w++] = (uint16_t)(q | (b << 6) | ((b < aq ? 1 : 0) << 8));
+                    if (conn[rank * nen + b] == node)
+                        ent[w++] = (uint32_t)(rank * nblk + ub(min(aq, b), max(aq, b), nen)) |
+                                   (node == r && b < aq ? 0x80000000u : 0u);
             }
         }
+        if (n > 0) last[r] = (uint16_t)w;
     }
     // column positions: rank of each valid column dof among the node's columns
     int L = 0;
@@ -428,59 +422,54 @@ __global__ void k_fill_nbrs(int64_t nnodes, int nen, int64_t n_mat, const int64_
     rowlen[r] = L;
 }
 
-// Per (node r, neighbour slot) the data the gather needs to compute each
-// node-block pair once: a block (r, s) with r < s is summed by r's warp,
-// which also writes it transposed into s's rows, when both nodes take the
-// gather's register path (a row of at most 64 or 128 positions, fewer than 32
-// neighbour slots, some row in the matrix); s's warp then skips it.  Per slot
-// one word: m << 4 | flags, flags bit 0 s < r, bit 1 s > r, bit 2 s qualifies
-// at 64 positions, bit 3 at 128; m, for s > r, the slot of r in s's list as an
-// index into the neighbour entries (6 m indexes colpos: the column positions
-// of r's dofs in s's rows).  lc: the row positions r's warp sums in the
-// register path of rows up to 64 positions (its row length less the columns
-// of lower neighbours that qualify there; 0 without rows).
-__global__ void k_slot_mirror(int64_t nnodes, int64_t n_mat, const int32_t *dof, const int64_t *nbr_off,
-                              const int32_t *nbr, const int32_t *rowlen, uint32_t *mir, int32_t *lc)
+// The blocks (r, s), s >= r, of node r for the value gather.  In a group of
+// GATHER_GROUP nodes the nodes' own blocks come first, then every node's
+// blocks with its higher neighbours in ascending order.
+__global__ void k_gather_items(int64_t nnodes, int nen, const int64_t *pp, const int64_t *nbr_off, const int32_t *nbr,
+                               const uint16_t *sl_off, const uint16_t *last, const uint32_t *src,
+                               const int64_t *item_off, GatherItem *items)
 {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nnodes) return;
-    const int64_t off = nbr_off[r], n = nbr_off[r + 1] - off;
-    bool rrow = false;
-    for (int k = 0; k < 6; k++) rrow |= dof[(int64_t)k * nnodes + r] <= n_mat;
-    const bool rq = rrow && n < 32 && rowlen[r] <= 64;
-    int cnt = rrow ? rowlen[r] : 0;
-    for (int64_t sl = 0; sl < n; sl++) {
-        const int32_t s = nbr[off + sl];
-        const int64_t so = nbr_off[s], sn = nbr_off[s + 1] - so;
-        int nfree = 0;
-        for (int k = 0; k < 6; k++) nfree += dof[(int64_t)k * nnodes + s] <= n_mat;
-        const bool anyrow = nfree > 0;
-        const int L = rowlen[s];
-        const bool q = anyrow && sn < 32;
-        if (rq && s < r && q && L <= 64) cnt -= nfree;
-        const uint32_t f = (s < r ? 1u : 0u) | (s > r ? 2u : 0u) | (q && L <= 64 ? 4u : 0u) | (q && L <= 128 ? 8u : 0u);
-        uint32_t mv = 0;
-        if (s > r) {
-            int64_t lo = 0, hi = sn - 1;  // r in s's sorted list
-            while (lo < hi) {
-                const int64_t mid = (lo + hi) >> 1;
-                if (nbr[so + mid] < r) lo = mid + 1; else hi = mid;
-            }
-            mv = (uint32_t)(so + lo);
-        }
-        mir[off + sl] = mv << 4 | f;
+    const int64_t g0 = r / GATHER_GROUP * GATHER_GROUP, ng = min((int64_t)GATHER_GROUP, nnodes - g0);
+    const int64_t own = item_off[g0] + (r - g0), first = item_off[r] - (r - g0) + ng - 1;
+    const int64_t off = nbr_off[r], n = nbr_off[r + 1] - off, p0 = pp[r] * nen;
+    if (n == 0) {
+        items[own] = GatherItem{(uint32_t)r, (uint32_t)r, 0, 0, 0, 0, 0, 0};
+        return;
     }
-    lc[r] = cnt;
+    const int64_t nup = item_off[r + 1] - item_off[r];
+    for (int64_t u = 0; u < nup; u++) {
+        const int64_t sl = n - nup + u;
+        const int32_t s = nbr[off + sl];
+        const int64_t so = nbr_off[s];
+        int64_t lo = 0, hi = nbr_off[s + 1] - so - 1;  // r in s's sorted list
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (nbr[so + mid] < r) lo = mid + 1; else hi = mid;
+        }
+        const int c0 = sl_off[off + sl], c1 = sl + 1 < n ? (int)sl_off[off + sl + 1] : (int)last[r];
+        GatherItem it;
+        it.r = (uint32_t)r;
+        it.s = (uint32_t)s;
+        it.k = (uint32_t)(off + sl);
+        it.m = (uint32_t)(so + lo);
+        it.cnt = (uint32_t)(c1 - c0);
+        it.e0 = src[p0 + c0];
+        it.e1 = c1 - c0 > 1 ? src[p0 + c0 + 1] : it.e0;
+        it.more = (uint32_t)(p0 + c0);
+        items[u == 0 ? own : first + u] = it;
+    }
 }
 
-// *out = max(v[0..n)) (out zeroed before; values are non-negative)
-__global__ void k_max_i32(int64_t n, const int32_t *v, int32_t *out)
+// where the row of each node's dof starts (-1: not in the matrix)
+__global__ void k_row_starts(int64_t nnodes, int64_t n_mat, const int32_t *dof, const int64_t *rowptr, int64_t *rowstart)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int32_t x = i < n ? v[i] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
-    if ((threadIdx.x & 31) == 0 && x > 0) atomicMax(out, x);
+    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= 6 * nnodes) return;
+    const int64_t r = q / 6;
+    const int32_t d = dof[(q - 6 * r) * nnodes + r];
+    rowstart[q] = d <= n_mat ? rowptr[d - 1] : -1;
 }
 
 __global__ void k_row_lengths(int64_t nnodes, int64_t n_mat, const int32_t *dof, const int32_t *rowlen,
@@ -539,9 +528,13 @@ int build_pattern(fs_ctx *c, int64_t n)
     int64_t nn = m.nnodes;
     if (n > 0x7fffffffLL) return set_err(c, FS_ERR_UNSUPPORTED, "matrix size above 2^31-1");
     int64_t *cnt = nullptr;
-    FS_TRY(grow(c, &P.tmp_cnt, &P.cap_tmp_cnt, (size_t)std::max<int64_t>(nn, n)));
+    FS_TRY(grow(c, &P.tmp_cnt, &P.cap_tmp_cnt, (size_t)std::max<int64_t>(2 * nn, n)));
     cnt = P.tmp_cnt;
-    if (nn) k_count_nbrs<<<nblk(nn, 128), 128, 0, c->stream>>>(nn, m.nen, m.pp, m.pair_e, m.conn, cnt, c->d_status);
+    if (nn)
+        k_count_nbrs<<<nblk(nn, 128), 128, 0, c->stream>>>(nn, m.nen, m.pp, m.pair_e, m.conn, cnt, cnt + nn,
+                                                           c->d_status);
+    FS_TRY(grow(c, &P.item_off, &P.cap_item_off, (size_t)nn + 1));
+    FS_TRY(exclusive_scan_i64(c, cnt + nn, P.item_off, nn, nullptr));
     FS_TRY(grow(c, &P.nbr_off, &P.cap_nbr_off, (size_t)nn + 1));
     int64_t nbr_total = 0;
     FS_TRY(exclusive_scan_i64(c, cnt, P.nbr_off, nn, &nbr_total));
@@ -551,16 +544,16 @@ int build_pattern(fs_ctx *c, int64_t n)
         return set_err(c, FS_ERR_UNSUPPORTED, "more than 255 neighbour nodes at one node");
     }
     FS_TRY(grow(c, &P.nbr, &P.cap_nbr, (size_t)nbr_total));
-    FS_TRY(grow(c, &P.pair_slots, &P.cap_pair_slots, (size_t)m.npairs));
     FS_TRY(grow(c, &P.colpos, &P.cap_colpos, (size_t)nbr_total * 6));
     FS_TRY(grow(c, &P.colsrc, &P.cap_colsrc, (size_t)nbr_total * 6));
     FS_TRY(grow(c, &P.rowlen, &P.cap_rowlen, (size_t)nn));
     FS_TRY(grow(c, &P.sl_off, &P.cap_sl_off, (size_t)nbr_total));
-    FS_TRY(grow(c, &P.sl_ent, &P.cap_sl_ent, (size_t)(m.npairs * m.nen)));
+    FS_TRY(grow(c, &P.sl_last, &P.cap_sl_last, (size_t)nn));
+    FS_TRY(grow(c, &P.src, &P.cap_src, (size_t)(m.npairs * m.nen)));
     if (nn)
         k_fill_nbrs<<<nblk(nn, 128), 128, 0, c->stream>>>(nn, m.nen, n, m.pp, m.pair_e, m.conn, m.dof, P.nbr_off,
-                                                         P.nbr, P.pair_slots, P.colpos, P.colsrc, P.rowlen,
-                                                         P.sl_off, P.sl_ent);
+                                                         P.nbr, P.colpos, P.colsrc, P.rowlen, P.sl_off, P.sl_last,
+                                                         P.src);
     // row lengths by dof
     int32_t *owner = nullptr;
     FS_TRY(grow(c, &P.tmp_owner, &P.cap_tmp_owner, (size_t)n));
@@ -568,46 +561,37 @@ int build_pattern(fs_ctx *c, int64_t n)
     FS_CUDA(c, cudaMemsetAsync(owner, 0, sizeof(int32_t) * std::max<int64_t>(n, 1), c->stream));
     FS_CUDA(c, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * std::max<int64_t>(n, 1), c->stream));
     if (nn) k_row_lengths<<<nblk(6 * nn, 256), 256, 0, c->stream>>>(nn, n, m.dof, P.rowlen, cnt, owner, c->d_status);
-    // longest row (selects the gather variant): reduced on the device, read
-    // back with the scan total
-    int32_t *d_max = reinterpret_cast<int32_t *>(owner);  // owner counts are consumed by k_row_lengths
-    FS_CUDA(c, cudaMemsetAsync(d_max, 0, sizeof(int32_t), c->stream));
-    if (nn) k_max_i32<<<nblk(nn, 256), 256, 0, c->stream>>>(nn, P.rowlen, d_max);
-    int32_t mx = 0;
-    FS_CUDA(c, cudaMemcpyAsync(&mx, d_max, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     FS_TRY(grow(c, &P.rowptr, &P.cap_rowptr, (size_t)n + 1));
     int64_t nnz = 0;
     FS_TRY(exclusive_scan_i64(c, cnt, P.rowptr, n, &nnz));
-    P.maxlen = mx;  // the scan's read-back synchronised the stream
+    FS_CUDA(c, cudaMemcpyAsync(&P.nitems, P.item_off + nn, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
     FS_TRY(read_status(c, &bits));
     if (bits & DEV_BAD_DOF) return set_err(c, FS_ERR_BAD_INPUT, "two dofs share one dof number");
     FS_TRY(grow(c, &P.colidx, &P.cap_colidx, (size_t)nnz));
     if (nn)
         k_fill_colidx<<<nblk(nn * 32, 256), 256, 0, c->stream>>>(nn, n, m.dof, P.nbr_off, P.nbr, P.colsrc,
                                                                   P.rowlen, P.rowptr, P.colidx);
-    // node-block pairs summed once (neighbour entry indices fit 28 bits)
-    P.maxlc = mx;
-    if (nbr_total < (1LL << 28)) {
-        FS_TRY(grow(c, &P.sl_mir, &P.cap_sl_mir, (size_t)nbr_total));
-        FS_TRY(grow(c, &P.lc, &P.cap_lc, (size_t)nn));
+    // the gather's list: 32-bit positions of neighbour entries and
+    // contributions, 31-bit ones of element blocks; a mesh beyond that (whose
+    // element matrices no device holds) keeps its pattern but has no gather
+    if (nbr_total < (1LL << 32) && m.npairs * m.nen < (1LL << 32) &&
+        m.nelem * n_upper_blocks(m.nen) < (1LL << 31)) {
+        FS_TRY(grow(c, &P.items, &P.cap_items, (size_t)P.nitems));
+        FS_TRY(grow(c, &P.rowstart, &P.cap_rowstart, (size_t)(6 * nn)));
         if (nn) {
-            k_slot_mirror<<<nblk(nn, 128), 128, 0, c->stream>>>(nn, n, m.dof, P.nbr_off, P.nbr, P.rowlen, P.sl_mir,
-                                                               P.lc);
-            // the longest summed row (selects the one-column variant of the gather)
-            FS_CUDA(c, cudaMemsetAsync(d_max, 0, sizeof(int32_t), c->stream));
-            k_max_i32<<<nblk(nn, 256), 256, 0, c->stream>>>(nn, P.lc, d_max);
-            FS_CUDA(c, cudaMemcpyAsync(&mx, d_max, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+            k_gather_items<<<nblk(nn, 128), 128, 0, c->stream>>>(nn, m.nen, m.pp, P.nbr_off, P.nbr, P.sl_off,
+                                                                 P.sl_last, P.src, P.item_off, P.items);
+            k_row_starts<<<nblk(6 * nn, 256), 256, 0, c->stream>>>(nn, n, m.dof, P.rowptr, P.rowstart);
         }
-        P.sym = true;
     } else {
-        P.sym = false;
+        dfree(&P.items);
+        P.cap_items = 0;
     }
     FS_TRY(grow(c, &P.diag_rowptr, &P.cap_diag_rowptr, (size_t)n + 1));
     FS_TRY(grow(c, &P.diag_colidx, &P.cap_diag_colidx, (size_t)n));
     k_diag_pattern<<<nblk(n + 1, 256), 256, 0, c->stream>>>(n, P.diag_rowptr, P.diag_colidx);
     FS_CUDA(c, cudaGetLastError());
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (P.sym && nn) P.maxlc = mx;
     P.n = n;
     P.nnz = nnz;
     return FS_OK;
