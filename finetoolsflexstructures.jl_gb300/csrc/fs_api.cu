@@ -217,6 +217,8 @@ int fs_ctx_destroy(fs_ctx *c)
     free_beam(c);
     free_shift(c);
     if (c->ke) cudaFree(c->ke);
+    if (c->fx_rows) cudaFree(c->fx_rows);
+    dfree(&c->fx_redo);
     dfree(&c->tmrm); dfree(&c->vals); dfree(&c->cmp_rowptr); dfree(&c->cmp_colidx); dfree(&c->cmp_vals);
     dfree(&c->stage64);
     if (c->scratch) cudaFree(c->scratch);
@@ -477,14 +479,17 @@ int fs::assemble_matrix(fs_ctx *c, int precision, int assembler, int64_t nrows, 
         FS_TRY(dalloc(c, &c->vals, need));
         c->vals_cap = need;
     }
-    if (beam_which < 0) FS_TRY(autotune_shell(c, precision));
-    FS_CUDA(c, cudaEventRecord(c->ev[0], c->stream));
-    FS_TRY(beam_which < 0 ? launch_elements(c, precision) : launch_beam_elements(c, beam_which, mass_type));
+    c->drops_zeros = assembler == FS_ASM_SPARSE_SYMM;
+    int st = beam_which < 0 ? autotune_shell(c, precision) : FS_OK;
+    if (st == FS_OK) st = cuda_check(c, cudaEventRecord(c->ev[0], c->stream), "cudaEventRecord");
+    if (st == FS_OK) st = beam_which < 0 ? launch_elements(c, precision) : launch_beam_elements(c, beam_which, mass_type);
+    c->drops_zeros = false;
+    FS_TRY(st);
     FS_CUDA(c, cudaEventRecord(c->ev[1], c->stream));
     FS_TRY(launch_gather(c, precision, c->vals));
     FS_CUDA(c, cudaEventRecord(c->ev[2], c->stream));
     int bits = 0;
-    FS_TRY(read_status(c, &bits));
+    FS_TRY(read_element_status(c, precision, c->ke, c->vals, &bits));
     FS_TRY(status_to_code(c, bits));
     c->timed = true;
     c->t_compact_ms = 0.0;
@@ -722,7 +727,7 @@ int fs_element_matrices(fs_ctx *c, int precision, double *out)
         return set_err(c, FS_ERR_STATE, "associategeometry! has not been called (self._associatedgeometry == true)");
     FS_TRY(launch_elements(c, precision));
     int bits = 0;
-    FS_TRY(read_status(c, &bits));
+    FS_TRY(read_element_status(c, precision, c->ke, nullptr, &bits));
     FS_TRY(status_to_code(c, bits));
     MeshDev &m = c->mesh;
     int nen = m.nen, nd = 6 * nen;

@@ -52,6 +52,14 @@ __device__ __forceinline__ void store_rows(R *o, const R (&acc)[NI][6])
     }
 }
 
+// three rows of a 6x6 block of doubles (16-byte stores)
+__device__ __forceinline__ void store_half(double *o, const double (&v)[3][6])
+{
+    double2 *o2 = reinterpret_cast<double2 *>(o);
+#pragma unroll
+    for (int q = 0; q < 9; q++) o2[q] = make_double2(v[q / 3][2 * (q % 3)], v[q / 3][2 * (q % 3) + 1]);
+}
+
 // One step of a compensated dot product (Ogita, Rump and Oishi's Dot2):
 // the product a*b is split exactly with an FMA and added to (s, c) by
 // TwoSum.  The _rn intrinsics are never contracted or reassociated.

@@ -1,0 +1,710 @@
+// FS_FP64 elements: geometry and strain coefficients in double, the expansion
+// to the global dofs and the Gram product in fixed point (fs_fixed.cuh).
+//
+// The rows are those of fs_elem_math.cuh (t3_rows, q4_point_rows) in two
+// steps.  First, in double, the coefficients of every row in the element frame:
+// u, v of a membrane row; w, the two rotations r0, r1 along the nodal triad's
+// first axes and the drilling multiplier mu of a bending or shear row, node by
+// node; and the largest magnitude of each kind.  Then, in fixed point, every row
+// is expanded in place: the coefficients with the element basis and the
+// nodal triads, whose entries are at most one, so that no row entry exceeds its
+// group by more than the expansion's own factor.  Row entries come in five
+// groups with an exponent each, for all rows and nodes of the element: the
+// translations of the membrane rows along each global axis (M), those of the
+// others (T), and the rotations (R).  An exponent for each axis keeps the small
+// components of an element near a coordinate plane: its membrane rows along the
+// normal must not disturb the much smaller bending stiffness there.
+#pragma once
+
+#include "fs_elem_math.cuh"
+#include "fs_fixed.cuh"
+
+#if defined(__CUDA_ARCH__)
+#define FS_UNROLL _Pragma("unroll")
+#define FS_ROLL _Pragma("unroll 1")
+#else
+#define FS_UNROLL
+#define FS_ROLL
+#endif
+
+namespace fs {
+
+// the symmetric-skew triad of a node (A10 = A01, A20 = -A02, A21 = -A12)
+struct Triad {
+    double a00, a01, a11, a02, a12, a22;
+};
+struct TriadFx {
+    fx a00, a01, a11, a02, a12, a22;
+};
+
+// Coefficient maxima (high words) of one element, and the exponents from them.
+struct FxMax {
+    uint32_t m = 0, w = 0, r = 0, u = 0, g = 0;  // u,v | w | r0,r1,drilling | mu | gradients
+    uint32_t e[3] = {0, 0, 0};                   // e0, e1 along each axis
+    FS_HD bool usable() const
+    {
+        return fx_usable(m) && fx_usable(w) && fx_usable(r) && fx_usable(u) && fx_usable(g);
+    }
+};
+struct FxExp {
+    int m[3], t, r;     // groups M (by axis), T and R
+    int em[3];          // units: e0, e1 along each axis
+    int cm;             // membrane coefficients
+    int u, g, h;        // mu, gradients, and the drilling coupling's h (u + g)
+    bool coupled;       // some mu is not zero
+};
+// spare: bits kept free for the longer sums of an element with several points
+FS_HD FxExp fx_exponents(const FxMax &mx, int spare)
+{
+    FxExp x;
+    x.cm = fx_exp(mx.m) + spare;
+    x.r = fx_exp(mx.r) + spare;
+    x.u = fx_exp(mx.u) + spare;
+    x.g = fx_exp(mx.g);
+    x.h = x.u + x.g;
+    x.coupled = mx.u != 0;
+    // |w e2 + sum h t| stays below 1.2 of the group: |w| below a half, |h| below
+    // three eighths in each component
+    const int w = fx_exp(mx.w);
+    x.t = (x.coupled && x.h + 2 > w ? x.h + 2 : w) + 1;
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) {
+        x.em[c] = fx_exp(mx.e[c]) > -60 ? fx_exp(mx.e[c]) : -60;  // below 2^-60 of the unit: counts as that
+        x.m[c] = x.cm + x.em[c];
+    }
+    return x;
+}
+
+// Nodal triad (nodal_triad), the drilling multipliers m0, m1 and the rotation
+// block R2 (symmetric) of build_map.
+FS_HD void triad_coefs(const double e[3][3], const double n[3], bool valid, Triad &A, double &m0, double &m1,
+                       double R2[3])
+{
+    double a0 = 0.0, a1 = 0.0;
+    if (valid) {
+        a0 = -dot3(e[1], n);
+        a1 = dot3(e[0], n);
+    }
+    const double x = a0 * a0 + a1 * a1;
+    if (!(x > 1.0e-24) && x == x) {
+        A = Triad{1.0, 0.0, 1.0, 0.0, 0.0, 1.0};
+        m0 = m1 = 0.0;
+        R2[0] = R2[2] = 1.0;
+        R2[1] = 0.0;
+        return;
+    }
+    double s, c;
+    sinc_cosc(x, s, c);
+    const double ca0 = c * a0, ca1 = c * a1;
+    A.a00 = 1.0 - ca1 * a1;
+    A.a01 = ca0 * a1;
+    A.a11 = 1.0 - ca0 * a0;
+    A.a02 = s * a1;
+    A.a12 = -(s * a0);
+    A.a22 = 1.0 - c * x;
+    const double inv = 1.0 / A.a22;
+    m0 = A.a02 * inv;
+    m1 = A.a12 * inv;
+    R2[0] = A.a00 - m0 * A.a02;
+    R2[1] = A.a01 - m0 * A.a12;
+    R2[2] = A.a11 - m1 * A.a12;
+}
+
+FS_HD TriadFx triad_fx(const Triad &A)
+{
+    return TriadFx{fx_make(A.a00, 0), fx_make(A.a01, 0), fx_make(A.a11, 0),
+                   fx_make(A.a02, 0), fx_make(A.a12, 0), fx_make(A.a22, 0)};
+}
+
+// t[k][c] = sum_r A[r][k] e[r][c]: the triad's axes in global components
+FS_HD void triad_axes(const TriadFx &A, const fx e[3][3], fx t[3][3])
+{
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) {
+        FxSum s = fx_mul(A.a00, e[0][c]);
+        fx_mac(s, A.a01, e[1][c]);
+        fx_mac(s, fx_neg(A.a02), e[2][c]);
+        t[0][c] = fx_done(s);
+        s = fx_mul(A.a01, e[0][c]);
+        fx_mac(s, A.a11, e[1][c]);
+        fx_mac(s, fx_neg(A.a12), e[2][c]);
+        t[1][c] = fx_done(s);
+        s = fx_mul(A.a02, e[0][c]);
+        fx_mac(s, A.a12, e[1][c]);
+        fx_mac(s, A.a22, e[2][c]);
+        t[2][c] = fx_done(s);
+    }
+}
+
+// One row slot of an element: a coefficient (double) before the expansion, a
+// row entry (fx) after it.  The slots of FX_GROUP elements lie interleaved, slot
+// by slot, so that the threads of a warp, an element each, touch contiguous
+// memory.
+union FxSlot {
+    double d;
+    fx x;
+};
+constexpr int FX_GROUP = 32;
+struct FxSlots {
+    FxSlot *p;
+    FS_HD FxSlot &operator[](int i) const { return p[i * FX_GROUP]; }
+    FS_HD FxSlots operator+(int i) const { return FxSlots{p + i * FX_GROUP}; }
+};
+
+// Membrane row in place: [u0 v0 u1 v1 ..] -> NN x 3 translations
+template <int NN> FS_HD void expand_membrane(FxSlots row, const fx em[2][3], int cm)
+{
+    fx u[NN], v[NN];
+    FS_UNROLL
+    for (int j = 0; j < NN; j++) {
+        u[j] = fx_make(row[2 * j].d, cm);
+        v[j] = fx_make(row[2 * j + 1].d, cm);
+    }
+    FS_UNROLL
+    for (int j = 0; j < NN; j++)
+        FS_UNROLL
+        for (int c = 0; c < 3; c++) {
+            FxSum s = fx_mul(u[j], em[0][c]);
+            fx_mac(s, v[j], em[1][c]);
+            row[3 * j + c].x = fx_done(s);
+        }
+}
+
+// Bending or shear row in place: [w0.. | r0 r1 per node | mu0..] -> NN x 6
+// (translations, rotations).  g: the basis gradients (exponent ex.g).
+template <int NN>
+FS_HD void expand_bending(FxSlots row, bool has_w, const fx e2[3], const fx t[NN][3][3], const TriadFx A[NN],
+                          const fx g[NN][2], const FxExp &ex)
+{
+    fx r0[NN], r1[NN], w[NN], h[NN][3];
+    FS_UNROLL
+    for (int j = 0; j < NN; j++) {
+        w[j] = fx{0, 0};
+        if (has_w) w[j] = fx_make(row[j].d, ex.t);
+        r0[j] = fx_make(row[NN + 2 * j].d, ex.r);
+        r1[j] = fx_make(row[NN + 2 * j + 1].d, ex.r);
+    }
+    if (ex.coupled) {
+        // P_r = sum_i mu_i A_i[r][:], h_j = (g_jx P_1 - g_jy P_0) / 2
+        fx P[2][3], mu[NN];
+        FS_UNROLL
+        for (int i = 0; i < NN; i++) mu[i] = fx_make(row[3 * NN + i].d, ex.u);
+        FxSum s[2][3];
+        FS_UNROLL
+        for (int i = 0; i < NN; i++) {
+            const fx a0[3] = {A[i].a00, A[i].a01, A[i].a02}, a1[3] = {A[i].a01, A[i].a11, A[i].a12};
+            FS_UNROLL
+            for (int k = 0; k < 3; k++) {
+                if (i == 0) {
+                    s[0][k] = fx_mul(mu[i], a0[k]);
+                    s[1][k] = fx_mul(mu[i], a1[k]);
+                } else {
+                    fx_mac(s[0][k], mu[i], a0[k]);
+                    fx_mac(s[1][k], mu[i], a1[k]);
+                }
+            }
+        }
+        FS_UNROLL
+        for (int k = 0; k < 3; k++) {
+            P[0][k] = fx_done(s[0][k]);
+            P[1][k] = fx_done(s[1][k]);
+        }
+        const int sh = ex.t - ex.h + 1;  // to the group's exponent, and the half
+        FS_UNROLL
+        for (int j = 0; j < NN; j++)
+            FS_UNROLL
+            for (int k = 0; k < 3; k++) {
+                FxSum q = fx_mul(g[j][0], P[1][k]);
+                fx_mac(q, fx_neg(g[j][1]), P[0][k]);
+                h[j][k] = fx_split(fx_shift(fx_round(q), sh));
+            }
+    }
+    FS_UNROLL
+    for (int j = 0; j < NN; j++)
+        FS_UNROLL
+        for (int c = 0; c < 3; c++) {
+            FxSum s{0, 0};
+            if (has_w) s = fx_mul(w[j], e2[c]);
+            if (ex.coupled)
+                FS_UNROLL
+                for (int k = 0; k < 3; k++) fx_mac(s, h[j][k], t[j][k][c]);
+            row[6 * j + c].x = fx_done(s);
+            s = fx_mul(r0[j], t[j][0][c]);
+            fx_mac(s, r1[j], t[j][1][c]);
+            row[6 * j + 3 + c].x = fx_done(s);
+        }
+}
+
+// What the expansion of an element (or Gauss point) needs beside its slots.
+template <int NN> struct FxGeom {
+    double e[3][3];    // element basis
+    Triad A[NN];
+    double g[NN][2];   // basis gradients
+};
+// maxima of the basis components
+template <int NN> FS_HD void fx_max_basis(FxMax &mx, const FxGeom<NN> &geo)
+{
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) {
+        fx_max(mx.e[c], geo.e[0][c]);
+        fx_max(mx.e[c], geo.e[1][c]);
+    }
+}
+
+// T3FF, homogeneous, average B: coefficients into the slots (CompactRows<3, 2>
+// layout).  In the element frame the first edge lies on x: with A, C, D its
+// length and the third node's coordinates, the averaged DSG shear rows
+// (_add_Bsmat_o! over the three node orderings) have the closed form below in
+// q = C/A, r = D/A, s = A/D.
+FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeom<3> &geo, FxMax &mx)
+{
+    typedef CompactRows<3, 2> L;
+    double J0[3], J1[3], (&e)[3][3] = geo.e;
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) {
+        J0[c] = in.X[1][c] - in.X[0][c];
+        J1[c] = in.X[2][c] - in.X[0][c];
+    }
+    const double n0 = dot3(J0, J0), ia = rsqrt_d(n0);
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) e[0][c] = J0[c] * ia;
+    cross3(e[0], J1, e[2]);
+    const double n2 = dot3(e[2], e[2]), id = rsqrt_d(n2);
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) e[2][c] *= id;
+    cross3(e[2], e[0], e[1]);
+    const double a = n0 * ia, d = n2 * id, q = dot3(J1, e[0]) * ia, r = d * ia, s = a * id;
+    const double Jd = a * d, t = in.t;
+    const double gx0 = -ia, gx1 = ia, gy0 = (q - 1.0) * id, gy1 = -(q * id), gy2 = id;
+    geo.g[0][0] = gx0; geo.g[0][1] = gy0;
+    geo.g[1][0] = gx1; geo.g[1][1] = gy1;
+    geo.g[2][0] = 0.0; geo.g[2][1] = gy2;
+    fx_max(mx.g, gx1);
+    fx_max(mx.g, gy0);
+    fx_max(mx.g, gy1);
+    fx_max(mx.g, gy2);
+    // weights: sqrt(t Ae), sqrt(t^3/12 Ae), sqrt(t stab Ae)
+    const double sm = sqrt(t * (0.5 * Jd)), sb = sm * t * 0.28867513459481288, ws = sm * t * rsqrt_d(t * t + mc.stab_c * Jd);
+    double R2[3][3], m0[3], m1[3];
+    FS_UNROLL
+    for (int i = 0; i < 3; i++) triad_coefs(e, in.nrm[i], in.valid[i], geo.A[i], m0[i], m1[i], R2[i]);
+    double ksum = 0.0;
+    // a bending or shear row's rotations tx, ty in the nodal triads
+    auto rotations = [&](FxSlots row, const double (&tx)[3], const double (&ty)[3]) {
+        FS_UNROLL
+        for (int j = 0; j < 3; j++) {
+            const double r0 = tx[j] * R2[j][0] + ty[j] * R2[j][1], r1 = tx[j] * R2[j][1] + ty[j] * R2[j][2];
+            const double mu = tx[j] * m0[j] + ty[j] * m1[j];
+            ksum += r0 * r0;
+            ksum += r1 * r1;
+            fx_max(mx.r, r0);
+            fx_max(mx.r, r1);
+            fx_max(mx.u, mu);
+            row[3 + 2 * j].d = r0;
+            row[4 + 2 * j].d = r1;
+            row[9 + j].d = mu;
+        }
+    };
+    // membrane and bending: the rows of L' (u,x  v,y  u,y + v,x)
+    auto membrane_bending = [&](int k, const double (&al)[3], const double (&be)[3]) {
+        const FxSlots mr = slot + L::MS * k;
+        double tx[3], ty[3];
+        FS_UNROLL
+        for (int j = 0; j < 3; j++) {
+            const double u = sm * be[j], v = sm * al[j];
+            fx_max(mx.m, u);
+            fx_max(mx.m, v);
+            mr[2 * j].d = u;
+            mr[2 * j + 1].d = v;
+            tx[j] = -(sb * al[j]);
+            ty[j] = sb * be[j];
+        }
+        rotations(slot + L::BS + L::BSS * k, tx, ty);
+    };
+    {
+        const double c0 = mc.Lps[lp(0, 0)], c1 = mc.Lps[lp(1, 0)], c2 = mc.Lps[lp(2, 0)];
+        const double al[3] = {c1 * gy0 + c2 * gx0, c1 * gy1 + c2 * gx1, c1 * gy2};
+        const double be[3] = {c0 * gx0 + c2 * gy0, c0 * gx1 + c2 * gy1, c2 * gy2};
+        membrane_bending(0, al, be);
+    }
+    {
+        const double c1 = mc.Lps[lp(1, 1)], c2 = mc.Lps[lp(2, 1)];
+        const double al[3] = {c1 * gy0 + c2 * gx0, c1 * gy1 + c2 * gx1, c1 * gy2};
+        const double be[3] = {c2 * gy0, c2 * gy1, c2 * gy2};
+        membrane_bending(1, al, be);
+    }
+    {
+        const double c2 = mc.Lps[lp(2, 2)];
+        const double al[3] = {c2 * gx0, c2 * gx1, 0.0};
+        const double be[3] = {c2 * gy0, c2 * gy1, c2 * gy2};
+        membrane_bending(2, al, be);
+    }
+    {
+        const double f0 = ws * mc.Lt[lp(0, 0)], f1 = ws * mc.Lt[lp(1, 0)], f2 = ws * mc.Lt[lp(1, 1)];
+        const double q6 = q * (1.0 / 6), r6 = r * (1.0 / 6), s6 = s * (1.0 / 6);
+        const double y0[3] = {1.0 / 3 + q6, 0.5 - q6, 1.0 / 6};                       // g_xz: thy
+        const double x1[3] = {q6 - 1.0 / 3, -(1.0 / 6) - q6, -0.5};                   // g_yz: thx
+        const double y1[3] = {s6 * (1.0 - q * q), s6 * q * (q - 2.0), s6 * (2.0 * q - 1.0)};  // g_yz: thy
+        FxSlots row = slot + L::BS + L::BSS * 3;
+        {
+            const double w[3] = {f0 * gx0 + f1 * gy0, f0 * gx1 + f1 * gy1, f1 * gy2};
+            const double tx[3] = {f1 * x1[0] - f0 * r6, f1 * x1[1] + f0 * r6, f1 * x1[2]};
+            const double ty[3] = {f0 * y0[0] + f1 * y1[0], f0 * y0[1] + f1 * y1[1], f0 * y0[2] + f1 * y1[2]};
+            FS_UNROLL
+            for (int j = 0; j < 3; j++) {
+                fx_max(mx.w, w[j]);
+                row[j].d = w[j];
+            }
+            rotations(row, tx, ty);
+        }
+        row = row + L::BSS;
+        const double w[3] = {f2 * gy0, f2 * gy1, f2 * gy2};
+        const double tx[3] = {f2 * x1[0], f2 * x1[1], f2 * x1[2]};
+        const double ty[3] = {f2 * y1[0], f2 * y1[1], f2 * y1[2]};
+        FS_UNROLL
+        for (int j = 0; j < 3; j++) {
+            fx_max(mx.w, w[j]);
+            row[j].d = w[j];
+        }
+        rotations(row, tx, ty);
+    }
+    // drilling factor: the mean of the nodal-basis bending diagonals
+    // (src/FEMMShellT3FFModule.jl:713-727)
+    const double sk = sqrt(ksum * mc.drill_scale6);
+    fx_max(mx.r, sk);
+    slot[L::DR].d = sk;
+    fx_max_basis(mx, geo);
+}
+
+// The membrane rows (MS apart) and the bending and shear rows (from BS, BSS
+// apart) of an element or Gauss point expanded in place; t: the nodal triads'
+// axes.
+template <int NN, int MS, int BS, int BSS>
+FS_HD void expand_slots(FxSlots slot, const FxGeom<NN> &geo, const FxExp &ex, fx t[NN][3][3])
+{
+    fx e[3][3];
+    {
+        fx em[2][3];
+        FS_UNROLL
+        for (int c = 0; c < 3; c++) {
+            em[0][c] = fx_make(geo.e[0][c], ex.em[c]);
+            em[1][c] = fx_make(geo.e[1][c], ex.em[c]);
+            FS_UNROLL
+            for (int k = 0; k < 3; k++) e[k][c] = fx_make(geo.e[k][c], 0);
+        }
+        FS_ROLL
+        for (int k = 0; k < 3; k++) expand_membrane<NN>(slot + MS * k, em, ex.cm);
+    }
+    fx g[NN][2];
+    TriadFx A[NN];
+    FS_UNROLL
+    for (int i = 0; i < NN; i++) {
+        A[i] = triad_fx(geo.A[i]);
+        triad_axes(A[i], e, t[i]);
+        g[i][0] = fx_make(geo.g[i][0], ex.g);
+        g[i][1] = fx_make(geo.g[i][1], ex.g);
+    }
+    FS_ROLL
+    for (int k = 0; k < 5; k++) expand_bending<NN>(slot + BS + BSS * k, k >= 3, e[2], t, A, g, ex);
+}
+
+// the slots of t3_coefs expanded in place, and the drilling rows
+FS_HD void t3_expand(FxSlots slot, const FxGeom<3> &geo, const bool valid[3], const FxExp &ex)
+{
+    typedef CompactRows<3, 2> L;
+    fx t[3][3][3];
+    expand_slots<3, L::MS, L::BS, L::BSS>(slot, geo, ex, t);
+    const fx sk = fx_make(slot[L::DR].d, ex.r);
+    FS_UNROLL
+    for (int i = 0; i < 3; i++)
+        FS_UNROLL
+        for (int c = 0; c < 3; c++) {
+            const FxSum s = fx_mul(sk, t[i][2][c]);
+            slot[L::DR + 3 * i + c].x = valid[i] ? fx_done(s) : fx{0, 0};
+        }
+}
+
+// Q4RS, homogeneous: coefficients of Gauss point j into its Q4Compact block,
+// and its share of the drilling traces (src/FEMMShellQ4RSModule.jl:807-838).
+// Xr: the nodes relative to the centroid; rn: 1 / |n| of the nodal normals (0
+// for a zero one); ss: square root of the stabilisation factor.  In the element
+// frame the first tangent lies on x, so that the MITC rows (_Bsmat) lose their
+// terms in its y component.  Returns nonzero on a singular metric.
+FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool valid[4], const double rn[4], double t,
+                   double ss, int j, const MatConst &mc, FxSlots slot, FxGeom<4> &geo, FxMax &mx, double trace[4])
+{
+    typedef Q4Compact L;
+    double gp[4][2], J0[3], J1[3], (&e)[3][3] = geo.e;
+    q4_dbasis_gp(j, gp);
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) {
+        J0[c] = Xr[0][c] * gp[0][0] + Xr[1][c] * gp[1][0] + Xr[2][c] * gp[2][0] + Xr[3][c] * gp[3][0];
+        J1[c] = Xr[0][c] * gp[0][1] + Xr[1][c] * gp[1][1] + Xr[2][c] * gp[2][1] + Xr[3][c] * gp[3][1];
+    }
+    const double n0 = dot3(J0, J0), ia = rsqrt_d(n0);
+    {
+        const double G12 = dot3(J0, J1), G22 = dot3(J1, J1);
+        if (n0 * G22 - G12 * G12 == 0.0) return 4;
+    }
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) e[0][c] = J0[c] * ia;
+    cross3(e[0], J1, e[2]);
+    const double n2 = dot3(e[2], e[2]), id = rsqrt_d(n2);
+    FS_UNROLL
+    for (int c = 0; c < 3; c++) e[2][c] *= id;
+    cross3(e[2], e[0], e[1]);
+    const double j11 = n0 * ia, j12 = dot3(J1, e[0]), j22 = n2 * id, q = j12 * ia;
+    double x[4], y[4];
+    FS_UNROLL
+    for (int a = 0; a < 4; a++) {
+        x[a] = dot3(Xr[a], e[0]);
+        y[a] = dot3(Xr[a], e[1]);
+        geo.g[a][0] = ia * gp[a][0];
+        geo.g[a][1] = id * (gp[a][1] - q * gp[a][0]);
+        fx_max(mx.g, geo.g[a][0]);
+        fx_max(mx.g, geo.g[a][1]);
+    }
+    // weights: sqrt(t Jac), sqrt(t^3/12 Jac), sqrt(t stab Jac)
+    const double sm = sqrt(t * (j11 * j22)), sb = sm * t * 0.28867513459481288, ws = sm * ss;
+    double R2[4][3], m0[4], m1[4], tn0[4], tn1[4];
+    FS_UNROLL
+    for (int i = 0; i < 4; i++) {
+        triad_coefs(e, nrm[i], valid[i], geo.A[i], m0[i], m1[i], R2[i]);
+        // the first two triad axes along the unit normal
+        const double c0 = dot3(e[0], nrm[i]) * rn[i], c1 = dot3(e[1], nrm[i]) * rn[i], c2 = dot3(e[2], nrm[i]) * rn[i];
+        const Triad &A = geo.A[i];
+        tn0[i] = A.a00 * c0 + A.a01 * c1 - A.a02 * c2;
+        tn1[i] = A.a01 * c0 + A.a11 * c1 - A.a12 * c2;
+        trace[i] = 0.0;
+    }
+    auto rotations = [&](FxSlots row, const double (&tx)[4], const double (&ty)[4]) {
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            const double r0 = tx[i] * R2[i][0] + ty[i] * R2[i][1], r1 = tx[i] * R2[i][1] + ty[i] * R2[i][2];
+            const double mu = tx[i] * m0[i] + ty[i] * m1[i], p = r0 * tn0[i] + r1 * tn1[i];
+            trace[i] += r0 * r0;
+            trace[i] += r1 * r1;
+            trace[i] -= p * p;
+            fx_max(mx.r, r0);
+            fx_max(mx.r, r1);
+            fx_max(mx.u, mu);
+            row[4 + 2 * i].d = r0;
+            row[5 + 2 * i].d = r1;
+            row[12 + i].d = mu;
+        }
+    };
+    auto membrane_bending = [&](int k, const double (&al)[4], const double (&be)[4]) {
+        const FxSlots mr = slot + L::MS * k;
+        double tx[4], ty[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            const double u = sm * be[i], v = sm * al[i];
+            fx_max(mx.m, u);
+            fx_max(mx.m, v);
+            mr[2 * i].d = u;
+            mr[2 * i + 1].d = v;
+            tx[i] = -(sb * al[i]);
+            ty[i] = sb * be[i];
+        }
+        rotations(slot + L::BS + L::BSS * k, tx, ty);
+    };
+    {
+        const double c0 = mc.Lps[lp(0, 0)], c1 = mc.Lps[lp(1, 0)], c2 = mc.Lps[lp(2, 0)];
+        double al[4], be[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            al[i] = c1 * geo.g[i][1] + c2 * geo.g[i][0];
+            be[i] = c0 * geo.g[i][0] + c2 * geo.g[i][1];
+        }
+        membrane_bending(0, al, be);
+    }
+    {
+        const double c1 = mc.Lps[lp(1, 1)], c2 = mc.Lps[lp(2, 1)];
+        double al[4], be[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            al[i] = c1 * geo.g[i][1] + c2 * geo.g[i][0];
+            be[i] = c2 * geo.g[i][1];
+        }
+        membrane_bending(1, al, be);
+    }
+    {
+        const double c2 = mc.Lps[lp(2, 2)];
+        double al[4], be[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            al[i] = c2 * geo.g[i][0];
+            be[i] = c2 * geo.g[i][1];
+        }
+        membrane_bending(2, al, be);
+    }
+    {
+        // tying lengths at the mirrored point: LA along x, LB along the second
+        // direction, whose unit vector is (j12, j22) / B
+        const double r = j < 2 ? -Q4_GP : Q4_GP, s = (j & 1) ? Q4_GP : -Q4_GP;
+        const double x01 = x[0] - x[1], x23 = x[2] - x[3], x03 = x[0] - x[3], x12 = x[1] - x[2];
+        const double y01 = y[0] - y[1], y23 = y[2] - y[3], y03 = y[0] - y[3], y12 = y[1] - y[2];
+        const double rp = r + 1.0, rm = r - 1.0, sp = s + 1.0, sm1 = s - 1.0;
+        const double ax = x01 * sp + x23 * sm1, ay = y01 * sp + y23 * sm1;
+        const double bx = x03 * rp - x12 * rm, by = y03 * rp - y12 * rm;
+        const double LA = sqrt(ax * ax + ay * ay), LB2 = bx * bx + by * by, B2 = j12 * j12 + j22 * j22;
+        const double d32 = ia * id * 0.03125, kb = LB2 * rsqrt_d(LB2 * B2) * d32;  // LB / B / (32 det)
+        const double q0 = j22 * kb, q1 = -(j12 * kb), p1 = -(LA * d32);
+        const double f0 = ws * mc.Lt[lp(0, 0)], f1 = ws * mc.Lt[lp(1, 0)], f2 = ws * mc.Lt[lp(1, 1)];
+        // node-wise factors of the two terms (w, thx, thy)
+        const double aw[4] = {2.0 * rp, -2.0 * rm, 2.0 * rm, -2.0 * rp}, bw[4] = {-2.0 * sp, 2.0 * sp, -2.0 * sm1, 2.0 * sm1};
+        const double axx[2] = {-(y03 * rp), y12 * rm}, axy[2] = {x03 * rp, -(x12 * rm)};    // nodes 0, 3 | 1, 2
+        const double bxx[2] = {y01 * sp, y23 * sm1}, bxy[2] = {-(x01 * sp), -(x23 * sm1)};  // nodes 0, 1 | 2, 3
+        double w1[4], x1[4], y1[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            const int ka = (i == 0 || i == 3) ? 0 : 1, kq = i < 2 ? 0 : 1;
+            w1[i] = p1 * aw[i] + q1 * bw[i];
+            x1[i] = p1 * axx[ka] + q1 * bxx[kq];
+            y1[i] = p1 * axy[ka] + q1 * bxy[kq];
+        }
+        const double g0 = f0 * q0;
+        FxSlots row = slot + L::BS + L::BSS * 3;
+        double tx[4], ty[4];
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            const int kq = i < 2 ? 0 : 1;
+            const double w = g0 * bw[i] + f1 * w1[i];
+            fx_max(mx.w, w);
+            row[i].d = w;
+            tx[i] = g0 * bxx[kq] + f1 * x1[i];
+            ty[i] = g0 * bxy[kq] + f1 * y1[i];
+        }
+        rotations(row, tx, ty);
+        row = row + L::BSS;
+        FS_UNROLL
+        for (int i = 0; i < 4; i++) {
+            const double w = f2 * w1[i];
+            fx_max(mx.w, w);
+            row[i].d = w;
+            tx[i] = f2 * x1[i];
+            ty[i] = f2 * y1[i];
+        }
+        rotations(row, tx, ty);
+    }
+    fx_max_basis(mx, geo);
+    return 0;
+}
+
+// 3 x 3 sums of products, and the pieces of a node block from them
+struct FxSums {
+    int64_t hh[3][3], c[3][3];
+    FS_HD void zero()
+    {
+        FS_UNROLL
+        for (int i = 0; i < 3; i++)
+            FS_UNROLL
+            for (int j = 0; j < 3; j++) hh[i][j] = c[i][j] = 0;
+    }
+    // entries (i, j), j >= i only on a diagonal block (UPPER)
+    template <bool UPPER> FS_HD void add(const fx (&a)[3], const fx *b)
+    {
+        FS_UNROLL
+        for (int i = 0; i < 3; i++)
+            FS_UNROLL
+            for (int j = UPPER ? i : 0; j < 3; j++) {
+                hh[i][j] += (int64_t)a[i].h * b[j].h;
+                c[i][j] += (int64_t)a[i].h * b[j].l;
+                c[i][j] += (int64_t)a[i].l * b[j].h;
+            }
+    }
+    FS_HD double value(int i, int j, int E) const { return fx_double(FxSum{hh[i][j], c[i][j]}, E); }
+};
+template <int N> FS_HD void fx_load(FxSlots p, fx (&v)[N])
+{
+    FS_UNROLL
+    for (int i = 0; i < N; i++) v[i] = p[i].x;
+}
+
+// One node block (p, q) of K from expanded rows: NP row sets (Gauss points),
+// `step` apart, of 3 membrane rows (MS apart, 3 values a node) and 5 bending and
+// shear rows (from BS, BSS apart, 6 values a node), and the node's drilling row
+// on a diagonal block.  top: rows 0..2 of the block into o, bottom: rows 3..5 (on a
+// diagonal block without its first three columns, the transpose of the top's
+// last three).
+template <int NP, int MS, int BS, int BSS, bool DIAG>
+FS_HD void fx_block_top(FxSlots rows, int step, int p, int q, const FxExp &ex, double o[3][6])
+{
+    FxSums m, tt, tr;
+    m.zero();
+    FS_ROLL
+    for (int pt = 0; pt < NP; pt++) {
+        FS_UNROLL
+        for (int k = 0; k < 3; k++) {
+            fx a[3], b[3];
+            fx_load(rows + pt * step + MS * k + 3 * p, a);
+            fx_load(rows + pt * step + MS * k + 3 * q, b);
+            m.template add<DIAG>(a, b);
+        }
+    }
+    FS_UNROLL
+    for (int i = 0; i < 3; i++)
+        FS_UNROLL
+        for (int j = DIAG ? i : 0; j < 3; j++) o[i][j] = m.value(i, j, ex.m[i] + ex.m[j]);
+    tt.zero();
+    tr.zero();
+    FS_ROLL
+    for (int pt = 0; pt < NP; pt++) {
+        FS_UNROLL
+        for (int k = 0; k < 5; k++) {
+            fx a[3], b[6];
+            fx_load(rows + pt * step + BS + BSS * k + 6 * p, a);
+            fx_load(rows + pt * step + BS + BSS * k + 6 * q, b);
+            tt.template add<DIAG>(a, b);
+            tr.template add<false>(a, b + 3);
+        }
+    }
+    FS_UNROLL
+    for (int i = 0; i < 3; i++) {
+        FS_UNROLL
+        for (int j = DIAG ? i : 0; j < 3; j++) {
+            o[i][j] += tt.value(i, j, 2 * ex.t);
+            if (DIAG && j > i) o[j][i] = o[i][j];
+        }
+        FS_UNROLL
+        for (int j = 0; j < 3; j++) o[i][3 + j] = tr.value(i, j, ex.t + ex.r);
+    }
+}
+template <int NP, int BS, int BSS, bool DIAG>
+FS_HD void fx_block_bottom(FxSlots rows, int step, int p, int q, FxSlots drill, const FxExp &ex,
+                           double o[3][6])
+{
+    FxSums rt, rr;
+    rt.zero();
+    rr.zero();
+    FS_ROLL
+    for (int pt = 0; pt < NP; pt++) {
+        FS_UNROLL
+        for (int k = 0; k < 5; k++) {
+            fx a[3], b[6];
+            fx_load(rows + pt * step + BS + BSS * k + 6 * p + 3, a);
+            fx_load(rows + pt * step + BS + BSS * k + 6 * q, b);
+            if (!DIAG) rt.template add<false>(a, b);
+            rr.template add<DIAG>(a, b + 3);
+        }
+    }
+    if (DIAG) {
+        fx d[3];
+        fx_load(drill, d);
+        rr.template add<true>(d, d);
+    }
+    FS_UNROLL
+    for (int i = 0; i < 3; i++) {
+        if (!DIAG) {
+            FS_UNROLL
+            for (int j = 0; j < 3; j++) o[i][j] = rt.value(i, j, ex.t + ex.r);
+        }
+        FS_UNROLL
+        for (int j = DIAG ? i : 0; j < 3; j++) {
+            o[i][3 + j] = rr.value(i, j, 2 * ex.r);
+            if (DIAG && j > i) o[j][3 + i] = o[i][3 + j];
+        }
+    }
+}
+
+}  // namespace fs

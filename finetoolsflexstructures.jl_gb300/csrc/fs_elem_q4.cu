@@ -35,8 +35,10 @@ size_t q4_smem(int precision, bool layered, int epb)
 
 // The elements per block (the tuned tile) is a launch parameter (block size
 // / 4): every tile runs the same compiled kernel and the same arithmetic.
+// only: null, or the elements to do (a byte each, by rank)
 template <class R, bool COMP, class S>
-__global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const MatConst mc, S *ke, int *status)
+__global__ void __launch_bounds__(128, 2)
+    k_q4_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
     constexpr int ND = 24;
     constexpr int RV = q4_row_values(COMP);
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const M
     Q4Stage &sg = reinterpret_cast<Q4Stage *>(smem_raw)[el];
     R *rows = reinterpret_cast<R *>(smem_raw + (size_t)epb * sizeof(Q4Stage) + (size_t)el * RB);
     const int64_t r = (int64_t)blockIdx.x * epb + el;
-    const bool active = r < m.nelem;
+    const bool active = r < m.nelem && (!only || only[r]);
     const int src = (threadIdx.x & 31) & ~3;  // the element's first lane
     // --- stage the element: lane qp loads node qp ---
     double Xa[3] = {0, 0, 0};
@@ -239,7 +241,7 @@ __global__ void __launch_bounds__(128, 2) k_q4_elements(const MeshDev m, const M
 }
 
 template <class R, bool COMP, class S = R>
-static int run_q4(fs_ctx *c, S *ke)
+static int run_q4(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
 {
     int epb = c->tune.elem_epb;
     if (epb != 8 && epb != 16 && epb != 32) epb = 16;
@@ -248,10 +250,13 @@ static int run_q4(fs_ctx *c, S *ke)
     const size_t smem = q4_smem(prec, COMP, epb);
     auto kern = k_q4_elements<R, COMP, S>;
     FS_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<nblk2(c->mesh.nelem, epb), epb * 4, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status);
+    kern<<<nblk2(c->mesh.nelem, epb), epb * 4, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status, only);
     FS_CUDA(c, cudaGetLastError());
     return FS_OK;
 }
+
+// the elements marked in `only` (null: all), in double
+int redo_q4(fs_ctx *c, double *ke, const uint8_t *only) { return run_q4<double, false>(c, ke, only); }
 
 // every Q4 variant: row precision, storage, layered
 int run_q4_any(fs_ctx *c, int precision, void *ke)
@@ -259,7 +264,8 @@ int run_q4_any(fs_ctx *c, int precision, void *ke)
     const bool comp = c->mesh.etype == FS_Q4RSCOMP;
     if (precision == FS_FP64) {
         double *k = (double *)ke;
-        return comp ? run_q4<double, true>(c, k) : run_q4<double, false>(c, k);
+        if (comp) return run_q4<double, true>(c, k);
+        return c->drops_zeros ? run_q4<double, false>(c, k) : run_fp64(c, k);
     }
     if (precision == FS_MIXED_COMP) {
         float2 *k = (float2 *)ke;

@@ -19,9 +19,10 @@ template <class R, bool COMP, bool AVGK, class S> struct T3MinBlocks {
     static constexpr int value = sizeof(R) == 8 ? 2 : (sizeof(S) == 8 ? (dense ? 2 : 3) : (dense ? 3 : 4));
 };
 
+// only: null, or the elements to do (a byte each, by rank)
 template <class R, bool COMP, bool AVGK, class S>
 __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
-    k_t3_elements(const MeshDev m, const MatConst mc, S *ke, int *status)
+    k_t3_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
     constexpr int NR = T3Rows<AVGK>::N, NS = T3Rows<AVGK>::NS;
     constexpr int ND = 18;
@@ -32,7 +33,7 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *rows = reinterpret_cast<R *>(smem_raw) + threadIdx.x * STRIDE;
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m.nelem) return;
+    if (r >= m.nelem || (only && !only[r])) return;
     ElemIn<3> in;
     load_elem<3>(m, r, in);
     const GroupConst *gc = COMP ? &m.groups[in.group] : nullptr;
@@ -46,7 +47,7 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
 }
 
 template <class R, bool COMP, bool AVGK, class S = R>
-static int run_t3(fs_ctx *c, S *ke)
+static int run_t3(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
 {
     int epb = c->tune.elem_epb;
     if (epb <= 0) epb = (sizeof(R) == 8 && AVGK) ? 64 : 128;
@@ -55,10 +56,13 @@ static int run_t3(fs_ctx *c, S *ke)
     const size_t smem = t3_smem(sizeof(R) == 8 ? FS_FP64 : FS_MIXED, AVGK, COMP, epb);
     auto kern = k_t3_elements<R, COMP, AVGK, S>;
     FS_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<nblk2(c->mesh.nelem, epb), epb, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status);
+    kern<<<nblk2(c->mesh.nelem, epb), epb, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status, only);
     FS_CUDA(c, cudaGetLastError());
     return FS_OK;
 }
+
+// the elements marked in `only` (null: all), in double
+int redo_t3(fs_ctx *c, double *ke, const uint8_t *only) { return run_t3<double, false, false>(c, ke, only); }
 
 // every T3 variant: row precision, storage, layered, average-K
 int run_t3_any(fs_ctx *c, int precision, void *ke)
@@ -68,7 +72,8 @@ int run_t3_any(fs_ctx *c, int precision, void *ke)
     if (precision == FS_FP64) {
         double *k = (double *)ke;
         if (comp) return avgk ? run_t3<double, true, true>(c, k) : run_t3<double, true, false>(c, k);
-        return avgk ? run_t3<double, false, true>(c, k) : run_t3<double, false, false>(c, k);
+        if (avgk) return run_t3<double, false, true>(c, k);
+        return c->drops_zeros ? run_t3<double, false, false>(c, k) : run_fp64(c, k);
     }
     if (precision == FS_MIXED_COMP) {
         float2 *k = (float2 *)ke;

@@ -28,7 +28,10 @@ enum : int {
     DEV_NEIGHBORS = 16,  // too many neighbour nodes
     DEV_BAD_ORDER = 32,
     DEV_NEG_DRILL = 64,
+    DEV_REDO = 128,      // elements marked for the double kernel (not an error)
 };
+
+static const unsigned NOALLOC_SCRATCH_BYTES = 32u << 20;  // element matrices of the allocation-free path
 
 static const int MAX_PAIRS_PER_NODE = 64;   // elements meeting at one node
 
@@ -137,6 +140,12 @@ struct fs_ctx {
     void *ke = nullptr;
     size_t ke_bytes = 0;
     double *tmrm = nullptr;
+    // FS_FP64: rows of a chunk of elements, and the elements to do in double
+    void *fx_rows = nullptr;
+    size_t cap_fx_rows = 0, fx_asked = 0;
+    bool drops_zeros = false;  // during an assembly that drops exact zeros
+    uint8_t *fx_redo = nullptr;
+    size_t cap_fx_redo = 0;
     // current matrix; mat_kind 0 a stiffness (shell or beam), 1 a mass, 2
     // another beam matrix
     int mat_kind = -1;
@@ -280,6 +289,11 @@ size_t t3_smem(int precision, bool avgk, bool layered, int epb);
 size_t entry_bytes(int precision);
 int run_t3_any(fs_ctx *c, int precision, void *ke);
 int run_q4_any(fs_ctx *c, int precision, void *ke);
+int run_fp64(fs_ctx *c, double *ke);
+int ensure_fp64_rows(fs_ctx *c);
+int redo_t3(fs_ctx *c, double *ke, const uint8_t *only);
+int redo_q4(fs_ctx *c, double *ke, const uint8_t *only);
+int read_element_status(fs_ctx *c, int precision, void *ke, double *vals, int *bits);
 size_t q4_smem(int precision, bool layered, int epb);
 
 // co-rotational beams

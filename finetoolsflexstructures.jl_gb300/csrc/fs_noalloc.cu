@@ -9,7 +9,7 @@
 // the element matrices (the only scratch of the assembly) in a fixed,
 // file-scope device array instead of a cudaMalloc'ed buffer.
 //
-// The array is FS_NOALLOC_SCRATCH_BYTES (32 MiB) on every GPU that loads the
+// The array is NOALLOC_SCRATCH_BYTES (32 MiB) on every GPU that loads the
 // library and stays there until the process exits.  Its device address is
 // looked up when a context is created (fs_ctx_create, with the context's
 // device current), so the library's device code and the array are loaded
@@ -21,11 +21,9 @@
 // be serialised by the caller.
 #include "fs_internal.cuh"
 
-#define FS_NOALLOC_SCRATCH_BYTES (32u << 20)
-
 namespace fs {
 
-static __device__ __align__(256) unsigned char fs_noalloc_scratch[FS_NOALLOC_SCRATCH_BYTES];
+static __device__ __align__(256) unsigned char fs_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
 // The array's address in the CUDA context current at context creation (the
 // context every buffer of `c` lives in).  A failed lookup is recorded, not
@@ -68,19 +66,19 @@ extern "C" int fs_stiffness_values_noalloc(fs_ctx *c, int precision, int64_t nro
     const int nen = c->mesh.nen;
     const uint64_t per = (uint64_t)n_upper_blocks(nen) * 36 * entry_bytes(precision);
     const uint64_t need = per * (uint64_t)c->mesh.nelem;
-    if (need > FS_NOALLOC_SCRATCH_BYTES) {
+    if (need > NOALLOC_SCRATCH_BYTES) {
         char msg[200];
         snprintf(msg, sizeof(msg),
                  "mesh too large for the allocation-free path: %lld elements need %llu bytes of element "
                  "matrices, the fixed scratch holds %u bytes (at most %llu elements)",
-                 (long long)c->mesh.nelem, (unsigned long long)need, (unsigned)FS_NOALLOC_SCRATCH_BYTES,
-                 (unsigned long long)(FS_NOALLOC_SCRATCH_BYTES / per));
+                 (long long)c->mesh.nelem, (unsigned long long)need, (unsigned)NOALLOC_SCRATCH_BYTES,
+                 (unsigned long long)(NOALLOC_SCRATCH_BYTES / per));
         return set_err(c, FS_ERR_UNSUPPORTED, msg);
     }
     if (!c->noalloc_scratch) return set_err(c, FS_ERR_CUDA, c->noalloc_err);
     FS_TRY(launch_elements_to(c, precision, c->noalloc_scratch));
     FS_TRY(launch_gather_from(c, precision, c->noalloc_scratch, vals));
     int bits = 0;
-    FS_TRY(read_status(c, &bits));
+    FS_TRY(read_element_status(c, precision, c->noalloc_scratch, vals, &bits));
     return status_to_code(c, bits);
 }

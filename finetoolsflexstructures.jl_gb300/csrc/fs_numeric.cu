@@ -8,10 +8,11 @@
 // forms K = Bh^T Bh as 6x6 node blocks.  The matrix is symmetric, so only its
 // upper node blocks (a <= b) are stored, by assembly rank, row-major inside a
 // block (6 of 9 blocks for T3, 10 of 16 for Q4); the gather reads a lower
-// block as the transpose of its mirror.
+// block as the transpose of its mirror.  The homogeneous elements in FS_FP64
+// have kernels of their own (fs_elem_fp64.cu).
 //
-// Gather.  Eighteen threads own one 6x6 block of the assembled matrix and add
-// the element blocks that touch it in ascending assembly rank, so every CSR
+// Gather.  Six threads own one 6x6 node-block pair of the assembled matrix and
+// add the element blocks that touch it in ascending assembly rank, so every CSR
 // value is the left-to-right sum of its element contributions in assembly
 // order, as Julia's sparse(I, J, V) combines duplicates.  No atomics: the
 // result is bitwise reproducible.
@@ -334,17 +335,19 @@ int launch_elements_to(fs_ctx *c, int precision, void *ke)
 // size of the gather (4, 8, 16 times 36 threads).  Each candidate is timed on the
 // context's own mesh with CUDA events (best of three launches), the element
 // kernel first, then the gather on its output.  The choice is keyed on
-// element family, precision, the average-K option and log2 of the element
-// count, and kept for the whole process.  Tile shapes change only how
+// element family, precision, the average-K option, whether exact zeros are
+// dropped (other kernels in FS_FP64) and log2 of the element count, and kept
+// for the whole process.  Tile shapes change only how
 // elements and nodes are grouped into blocks, never the arithmetic of one
 // element or one stored value, so every candidate gives bitwise the same
 // matrix.
 namespace {
 struct TuneKey {
-    int etype, precision, avgk, bucket;
+    int etype, precision, avgk, drops_zeros, bucket;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(etype, precision, avgk, bucket) < std::tie(o.etype, o.precision, o.avgk, o.bucket);
+        return std::tie(etype, precision, avgk, drops_zeros, bucket) <
+               std::tie(o.etype, o.precision, o.avgk, o.drops_zeros, o.bucket);
     }
 };
 std::mutex g_tune_mu;
@@ -392,7 +395,7 @@ int autotune_shell(fs_ctx *c, int precision)
     const bool avgk = c->params.transv_shear_formulation == 1;
     int bucket = 0;
     while ((int64_t(1) << (bucket + 1)) <= m.nelem) bucket++;
-    const TuneKey key{m.etype, precision, avgk ? 1 : 0, bucket};
+    const TuneKey key{m.etype, precision, avgk ? 1 : 0, c->drops_zeros ? 1 : 0, bucket};
     if (c->tune.mode == 1) {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune.find(key);

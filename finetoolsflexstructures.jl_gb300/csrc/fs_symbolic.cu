@@ -525,6 +525,9 @@ int build_pattern(fs_ctx *c, int64_t n)
     MeshDev &m = c->mesh;
     PatternDev &P = c->pat;
     if (P.n == n && P.rowptr) return FS_OK;
+    // a mesh that fits the allocation-free path has its row buffer from the start
+    if ((uint64_t)m.nelem * n_upper_blocks(m.nen) * 36 * sizeof(double) <= NOALLOC_SCRATCH_BYTES)
+        FS_TRY(ensure_fp64_rows(c));
     int64_t nn = m.nnodes;
     if (n > 0x7fffffffLL) return set_err(c, FS_ERR_UNSUPPORTED, "matrix size above 2^31-1");
     int64_t *cnt = nullptr;

@@ -46,7 +46,7 @@ extern "C" {
 #define FS_COROTBEAM 4  /* FEMMCorotBeam (2-node L2 beams), src/FEMMCorotBeamModule.jl */
 
 /* arithmetic of the element strain rows and Gram products */
-#define FS_FP64 0       /* everything in double: the drop-in                 */
+#define FS_FP64 0       /* double precision: the drop-in                     */
 #define FS_MIXED 1      /* float element arithmetic on element frames and
                            coordinates formed in double (the Q4 Gauss-point
                            frames and drilling factor in float); CSR values
