@@ -29,6 +29,8 @@ enum : int {
     DEV_BAD_ORDER = 32,
     DEV_NEG_DRILL = 64,
     DEV_REDO = 128,      // elements marked for the double kernel (not an error)
+    DEV_UNSYMMETRIC = 256,  // explicit set-up: K is not symmetric (not an error)
+    DEV_UNOWNED = 512,      // explicit set-up: a dof that no node has (not an error)
 };
 
 static const unsigned NOALLOC_SCRATCH_BYTES = 32u << 20;  // element matrices of the allocation-free path
@@ -193,11 +195,14 @@ struct fs_ctx {
         // 6x6 node-block form of K (block rows = the pattern's neighbour lists)
         bool bsr = false;
         int64_t nnodes = 0;
-        void *blk = nullptr;          // nbr_total x 36 (float or double)
+        int sms = 1;
+        bool one_pass = false;        // a step does the next one's displacement update too
+        void *item = nullptr;         // the rows' blocks (CdItem), by the pattern's neighbour lists
+        void *blk = nullptr;          // 36 values a block (float or double)
         void *res = nullptr;          // FS_MIXED_COMP: the rounding residual of the float
                                       // values (K - float(K)) in bf16, same layout as blk
                                       // (block form) or vals32 (CSR form)
-        void *xp = nullptr;           // displacement copy, 6 per node (float or double)
+        void *xp = nullptr;           // two displacement copies, 6 per node (double, float or float pairs)
         int32_t *pad_of_dof = nullptr;  // dof -> node * 6 + component
         bool ready = false;
         cudaGraph_t graph = nullptr;
