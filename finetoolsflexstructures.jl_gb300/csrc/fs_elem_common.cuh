@@ -183,9 +183,6 @@ template <int NI, int LEVELS = 3> struct PairAcc {
 };
 template <int NI> struct BlockAcc<float, true, NI> : PairAcc<NI, Q4_PAIR_LEVELS> {};
 
-// acc += sum over rows [r0, r1) of row[6a + i] row[6b + j] for i in
-// [I0, I1), j in [J0, J1): the sub-blocks a row can reach (DIAG: a = b, the
-// upper triangle)
 // The row loop of the gram helpers: unrolled, or (ROLLED) kept a loop.  The
 // T3 kernel's float-pair sums run rolled: a row's body is 16 packed
 // instructions per entry pair, and the unrolled loops stalled it on
@@ -201,23 +198,9 @@ __device__ __forceinline__ void for_rows(int r0, int r1, F body)
     }
 }
 
-template <int I0, int I1, int J0, int J1, bool DIAG = false, bool ROLLED = false, class R, class Acc>
-__device__ __forceinline__ void gram_rows(Acc &acc, const R *rows, int ND, int r0, int r1, int a, int b)
-{
-    for_rows<ROLLED>(r0, r1, [&](int rho) {
-        const R *rr = rows + rho * ND;
-        R ra[6], rb[6];
-#pragma unroll
-        for (int i = I0; i < I1; i++) ra[i] = rr[6 * a + i];
-#pragma unroll
-        for (int j = J0; j < J1; j++) rb[j] = rr[6 * b + j];
-        acc.template row<I0, I1, J0, J1, DIAG>(ra, rb);
-    });
-}
-
 // acc += sum over rows [r0, r1) (stride RS from base) of row[NSTR a + i - IOFF]
-// row[NSTR b + j - IOFF] for i in [I0, I1), j in [J0, J1): the same products
-// as gram_rows on a compact row layout (rows holding a subset of the dofs)
+// row[NSTR b + j - IOFF] for i in [I0, I1), j in [J0, J1): the sub-blocks that
+// a row can reach (DIAG: a = b, the upper triangle)
 template <int I0, int I1, int J0, int J1, int RS, int NSTR, int IOFF, bool DIAG = false, bool ROLLED = false,
           class R, class Acc>
 __device__ __forceinline__ void gram_rows_c(Acc &acc, const R *base, int r0, int r1, int a, int b)
@@ -303,8 +286,7 @@ __device__ __forceinline__ void for_upper_blocks(unsigned swapped, D diag, O off
 }
 
 // Upper node blocks of a homogeneous element from its rows in the
-// CompactRows<NN, NS> layout: the products and their order are those of the
-// SPARSE path of write_blocks, so the blocks are bitwise the same.
+// CompactRows<NN, NS> layout.
 template <class R, class S, int NN, int NS>
 __device__ __forceinline__ void write_blocks_compact(const R *rows, unsigned swapped, S *out)
 {
@@ -328,39 +310,25 @@ __device__ __forceinline__ void write_blocks_compact(const R *rows, unsigned swa
         });
 }
 
-// Upper node blocks of K = sum_rho row_rho row_rho^T.  Storage S: the row
-// type R itself, or float2 pairs for float rows accumulated in compensated
-// sums (FS_MIXED_COMP).  SPARSE (homogeneous shells): rows 0..2 are membrane rows
-// (nodal translations only) and the last NN rows drilling rows (the
-// rotations of one node each); their structurally zero products are
-// skipped, in the same row order, so the sums are those of the dense loop.
-template <class R, class S, int NN, bool SPARSE>
-__device__ __forceinline__ void write_blocks(const R *rows, int nrows, unsigned swapped, S *out)
+// Upper node blocks of a layered element from its rows in the LayeredRows<NN,
+// NR> layout
+template <class R, class S, int NN, int NR>
+__device__ __forceinline__ void write_blocks_layered(const R *rows, unsigned swapped, S *out)
 {
+    typedef LayeredRows<NN, NR> L;
     constexpr bool PAIR = sizeof(S) == 8 && sizeof(R) == 4;
-    const int ND = 6 * NN;
     for_upper_blocks<NN, PAIR>(
         swapped, [&](int a) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
-            if (SPARSE) {
-                gram_rows<0, 3, 0, 3, true, PAIR>(acc, rows, ND, 0, 3, a, a);
-                gram_rows<0, 6, 0, 6, true, PAIR>(acc, rows, ND, 3, nrows - NN, a, a);
-                gram_rows<3, 6, 3, 6, true, PAIR>(acc, rows, ND, nrows - NN + a, nrows - NN + a + 1, a, a);
-            } else {
-                gram_rows<0, 6, 0, 6, true, PAIR>(acc, rows, ND, 0, nrows, a, a);
-            }
+            gram_rows_c<0, 6, 0, 6, L::RS, 6, 0, true, PAIR>(acc, rows, 0, NR, a, a);
+            gram_rows_c<3, 6, 3, 6, 3, 0, 3, true, PAIR>(acc, rows + L::DR + 3 * a, 0, 1, a, a);
             acc.template store<true>(out + ub(a, a, NN) * 36);
         },
         [&](int a, int b, int o) {
             typename T3Acc<R, PAIR>::type acc;
             acc.zero();
-            if (SPARSE) {
-                gram_rows<0, 3, 0, 3, false, PAIR>(acc, rows, ND, 0, 3, a, b);
-                gram_rows<0, 6, 0, 6, false, PAIR>(acc, rows, ND, 3, nrows - NN, a, b);
-            } else {
-                gram_rows<0, 6, 0, 6, false, PAIR>(acc, rows, ND, 0, nrows, a, b);
-            }
+            gram_rows_c<0, 6, 0, 6, L::RS, 6, 0, false, PAIR>(acc, rows, 0, NR, a, b);
             acc.store(out + o * 36);
         });
 }

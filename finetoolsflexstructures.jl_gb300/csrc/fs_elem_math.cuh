@@ -450,22 +450,6 @@ struct GroupConst {
 };
 
 
-// rows_out[r] = scale * sum_{c>=r} L[c][r] rows_in[c]   (L^T applied to stacked rows)
-template <class R, int NN, int NR>
-FS_HD void mix_rows(const double *Lpk, const float *Lpkf, R scale, const R in[NR][NN][5], R out[NR][NN][5])
-{
-    for (int r = 0; r < NR; r++) {
-        R f[NR];
-        for (int c = 0; c < NR; c++) f[c] = (c >= r) ? scale * lpk<R>(Lpk, Lpkf, lp(c, r)) : (R)0;
-        for (int i = 0; i < NN; i++)
-            for (int q = 0; q < 5; q++) {
-                R s = 0;
-                for (int c = r; c < NR; c++) s += f[c] * in[c][i][q];
-                out[r][i][q] = s;
-            }
-    }
-}
-
 // Layup-to-element angle (reference Layup2ElementAngle, src/TransformerModule.jl:92-105)
 FS_HD void layup_angle(const double e[3][3], const double cs[9], double &m, double &n)
 {
@@ -482,30 +466,125 @@ FS_HD void layup_angle(const double e[3][3], const double cs[9], double &m, doub
     n = (nn >= 0.0 ? 1.0 : -1.0) * sqrt(q > 0.0 ? q : 0.0);
 }
 
-// Rotate the membrane and bending element-frame rows by Tbar and the shear
-// rows by Tts (plane_stress_Tbar_matrix!, src/CompositeLayupModule.jl:364-378;
-// transverse_shear_T_matrix!, :463-471): strain' = T strain.
+// Strain rows of a layered element, one at a time and straight to the global
+// dofs.  The membrane and bending strains are rotated by Tbar
+// (plane_stress_Tbar_matrix!, src/CompositeLayupModule.jl:364-378) and the
+// shear ones by Tts (transverse_shear_T_matrix!, :463-471): strain' = T strain.
+// With the gradient g of a node, the membrane rows are (g0, 0, g1) on u and
+// (0, g1, g0) on v, the bending rows the same on thy and, negated, on thx, so
+// their rotated values are held once: a[k][i] on u and thy, b[k][i] on v and
+// -thx.  Every row is formed in registers; with arrays of all of them, zeros
+// included, in local memory (1.2 to 1.8 KB a thread) the layered kernels spent most of their time
+// waiting for it: Q4RSComp, 300 x 256, a whole assembly in FS_MIXED_COMP 1279 us, now 630,
+// FS_FP64 5928 and 3333; T3FFComp 547 and 260, 1771 and 1064.
 template <class R, int NN>
-FS_HD void rotate3(double m, double n, R rows[3][NN][5])
+FS_HD void rotated_gradients(double m, double n, const R g[NN][2], R a[3][NN], R b[3][NN])
 {
-    double T[3][3] = {{m * m, n * n, -(m * n)}, {n * n, m * m, (m * n)}, {2 * (m * n), -2 * (m * n), m * m - n * n}};
-    for (int i = 0; i < NN; i++)
-        for (int q = 0; q < 5; q++) {
-            R a = rows[0][i][q], b = rows[1][i][q], c = rows[2][i][q];
-            rows[0][i][q] = (R)T[0][0] * a + (R)T[0][1] * b + (R)T[0][2] * c;
-            rows[1][i][q] = (R)T[1][0] * a + (R)T[1][1] * b + (R)T[1][2] * c;
-            rows[2][i][q] = (R)T[2][0] * a + (R)T[2][1] * b + (R)T[2][2] * c;
+    const double T[3][3] = {{m * m, n * n, -(m * n)}, {n * n, m * m, (m * n)}, {2 * (m * n), -2 * (m * n), m * m - n * n}};
+    for (int k = 0; k < 3; k++)
+        for (int i = 0; i < NN; i++) {
+            a[k][i] = fma((R)T[k][2], g[i][1], (R)T[k][0] * g[i][0]);
+            b[k][i] = fma((R)T[k][2], g[i][0], (R)T[k][1] * g[i][1]);
         }
 }
+
+// sum_{c >= r} f[c] x[c][i], c from 0 to 2 (f[c] = 0 for c < r)
 template <class R, int NN>
-FS_HD void rotate2(double m, double n, R rows[2][NN][5])
+FS_HD R mixed3(const R f[3], const R x[3][NN], int i)
 {
-    for (int i = 0; i < NN; i++)
-        for (int q = 0; q < 5; q++) {
-            R a = rows[0][i][q], b = rows[1][i][q];
-            rows[0][i][q] = (R)m * a - (R)n * b;
-            rows[1][i][q] = (R)n * a + (R)m * b;
+    return fma(f[2], x[2][i], fma(f[1], x[1][i], f[0] * x[0][i]));
+}
+
+// A row with in-plane translations u, v (HAS_UV), w (HAS_W) and rotations tx, ty
+// per node on the global dofs (expand_row without the absent terms).  The sums
+// of two products are written as the fused operations that plain code is
+// compiled to, so that a row does not depend on what surrounds it.
+template <class R, int NN, bool HAS_UV, bool HAS_W>
+FS_HD void expand_some(const GlobalMap<R, NN> &M, const R u[NN], const R v[NN], const R w[NN], const R tx[NN],
+                       const R ty[NN], R *out)
+{
+    R P0[3] = {0, 0, 0}, P1[3] = {0, 0, 0};
+    for (int i = 0; i < NN; i++) {
+        R mu = fma(tx[i], M.m[i][0], ty[i] * M.m[i][1]);
+        for (int k = 0; k < 3; k++) {
+            P0[k] += mu * M.A01[i][0][k];
+            P1[k] += mu * M.A01[i][1][k];
         }
+    }
+    for (int j = 0; j < NN; j++) {
+        R h[3];
+        for (int k = 0; k < 3; k++) h[k] = (R)0.5 * (M.g[j][0] * P1[k] - M.g[j][1] * P0[k]);
+        R r0 = fma(tx[j], M.R2[j][0][0], ty[j] * M.R2[j][1][0]);
+        R r1 = fma(tx[j], M.R2[j][0][1], ty[j] * M.R2[j][1][1]);
+        for (int q = 0; q < 3; q++) {
+            R s;
+            if constexpr (HAS_UV)
+                s = fma(h[0], M.t[j][0][q], fma(u[j], M.e[0][q], v[j] * M.e[1][q]));
+            else if constexpr (HAS_W)
+                s = fma(h[0], M.t[j][0][q], w[j] * M.e[2][q]);
+            else
+                s = h[0] * M.t[j][0][q];
+            out[6 * j + q] = fma(h[2], M.t[j][2][q], fma(h[1], M.t[j][1][q], s));
+            out[6 * j + 3 + q] = fma(r0, M.t[j][0][q], r1 * M.t[j][1][q]);
+        }
+    }
+}
+
+// Compact rows of a layered element: NR dense rows (6 NN values), then the drilling
+// rows (the 3 rotations of one node each).  Offsets in R units.
+template <int NN, int NR> struct LayeredRows {
+    static constexpr int RS = 6 * NN;
+    static constexpr int DR = NR * RS;
+    static constexpr int SIZE = DR + 3 * NN;
+};
+
+// The six membrane and bending rows (stride rs), mixed with the 6x6 factor of
+// [A B; B D]: row r = scale sum_{c >= r} L[c][r] strain_c.  Rows 3 to 5 have no
+// u and v.  rot(r, tx, ty): each row's rotations.
+template <class R, int NN, class F>
+FS_HD void layered_mb_rows(const GlobalMap<R, NN> &M, const GroupConst *gc, double m, double n, R scale, R *rows, int rs, F rot)
+{
+    R a[3][NN], b[3][NN];
+    rotated_gradients<R, NN>(m, n, M.g, a, b);
+    for (int r = 0; r < 6; r++) {
+        R f[6], u[NN], v[NN], tx[NN], ty[NN];
+        for (int c = 0; c < 6; c++) f[c] = c >= r ? scale * lpk<R>(gc->L6, gc->L6f, lp(c, r)) : (R)0;
+        for (int i = 0; i < NN; i++) {
+            tx[i] = -mixed3<R, NN>(f + 3, b, i);
+            ty[i] = mixed3<R, NN>(f + 3, a, i);
+        }
+        if (r < 3) {
+            for (int i = 0; i < NN; i++) {
+                u[i] = mixed3<R, NN>(f, a, i);
+                v[i] = mixed3<R, NN>(f, b, i);
+            }
+            expand_some<R, NN, true, false>(M, u, v, nullptr, tx, ty, rows + r * rs);
+        } else
+            expand_some<R, NN, false, false>(M, nullptr, nullptr, nullptr, tx, ty, rows + r * rs);
+        rot(r, tx, ty);
+    }
+}
+
+// Two shear rows (w, thx, thy of sh in the element frame), rotated and mixed
+// with the factor of H
+template <class R, int NN, class F>
+FS_HD void layered_shear_rows(const GlobalMap<R, NN> &M, const GroupConst *gc, double m, double n, R scale,
+                              const R (*sh)[NN][5], R *rows, int rs, F rot)
+{
+    const R f00 = scale * lpk<R>(gc->LH, gc->LHf, lp(0, 0)), f10 = scale * lpk<R>(gc->LH, gc->LHf, lp(1, 0)),
+            f11 = scale * lpk<R>(gc->LH, gc->LHf, lp(1, 1));
+    R x[2][3][NN];
+    for (int i = 0; i < NN; i++)
+        for (int q = 0; q < 3; q++) {
+            const R a = sh[0][i][2 + q], b = sh[1][i][2 + q];
+            const R p = (R)m * a - (R)n * b, s = (R)n * a + (R)m * b;
+            x[0][q][i] = fma(f10, s, f00 * p);
+            x[1][q][i] = f11 * s;
+        }
+    for (int r = 0; r < 2; r++) {
+        expand_some<R, NN, false, true>(M, nullptr, nullptr, x[r][0], x[r][1], x[r][2], rows + r * rs);
+        rot(r, x[r][1], x[r][2]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -546,11 +625,11 @@ FS_HD void t3_bs_ordering(const R x[3], const R y[3], R Ae, int s, int p, int q,
 
 // Computes the Gram rows (global dofs, 18 wide) of one T3FF / T3FFComp
 // element.  Returns 0 on success.  `rows` is written with row stride `rs`,
-// or (COMPACT, homogeneous elements) in the CompactRows<3, NS> layout.
+// or (COMPACT) in the CompactRows<3, NS> (homogeneous) or LayeredRows<3, 6 +
+// NS> layout (rs = 18).
 template <class R, bool COMP, bool AVGK, bool COMPACT = false>
 FS_HD int t3_rows(const ElemIn<3> &in, const MatConst &mc, const GroupConst *gc, R *rows, int rs)
 {
-    static_assert(!(COMP && COMPACT), "the compact layout is for homogeneous elements");
     // --- frame and element coordinates (double) ---
     double J0[3], J1[3], e[3][3];
     for (int c = 0; c < 3; c++) {
@@ -645,45 +724,46 @@ FS_HD int t3_rows(const ElemIn<3> &in, const MatConst &mc, const GroupConst *gc,
     } else {
         // --- layered: membrane and bending rows rotated by the layup angle and
         //     mixed with the 6x6 [A B; B D] factor, shear with H ---
-        R mb[6][3][5];
-        for (int r = 0; r < 6; r++)
-            for (int i = 0; i < 3; i++)
-                for (int q = 0; q < 5; q++) mb[r][i][q] = 0;
-        for (int i = 0; i < 3; i++) {
-            mb[0][i][0] = g[i][0];
-            mb[1][i][1] = g[i][1];
-            mb[2][i][0] = g[i][1]; mb[2][i][1] = g[i][0];
-            mb[3][i][4] = g[i][0];
-            mb[4][i][3] = -g[i][1];
-            mb[5][i][3] = -g[i][0]; mb[5][i][4] = g[i][1];
-        }
-        R mixed[6 + NS][3][5];
         double lm, ln;
         layup_angle(e, gc->csmat, lm, ln);
-        rotate3<R, 3>(lm, ln, (R(*)[3][5])mb[0]);
-        rotate3<R, 3>(lm, ln, (R(*)[3][5])mb[3]);
-        mix_rows<R, 3, 6>(gc->L6, gc->L6f, sqrt(AeR), mb, (R(*)[3][5])mixed[0]);
-        R ws = stab * AeR * (R)(AVGK ? 1.0 / 3 : 1.0);
-        for (int o = 0; o < NS / 2; o++) {
-            rotate2<R, 3>(lm, ln, (R(*)[3][5])sh[2 * o]);
-            mix_rows<R, 3, 2>(gc->LH, gc->LHf, sqrt(ws), (R(*)[3][5])sh[2 * o], (R(*)[3][5])mixed[6 + 2 * o]);
-        }
-        for (int r = 0; r < 6 + NS; r++) expand_row<R, 3>(M, (const R(*)[5])mixed[r], rows + r * rs);
-        // drilling factor: every mixed row may carry rotations here
-        R ksumr = 0;
-        for (int i = 0; i < 3; i++)
-            for (int cl = 0; cl < 2; cl++)
-                for (int r = 0; r < 6 + NS; r++) {
-                    R v = mixed[r][i][3] * M.R2[i][0][cl] + mixed[r][i][4] * M.R2[i][1][cl];
-                    ksumr += v * v;
+        // drilling factor: every row may carry rotations here.  Float rows: one
+        // running sum over the nodes, directions and then rows; double rows as
+        // the rows come
+        R ltx[sizeof(R) == 4 ? 6 + NS : 1][3], lty[sizeof(R) == 4 ? 6 + NS : 1][3], ksumr = 0;
+        auto add = [&](int r, const R *tx, const R *ty) {
+            for (int i = 0; i < 3; i++) {
+                if constexpr (sizeof(R) == 4) {
+                    ltx[r][i] = tx[i];
+                    lty[r][i] = ty[i];
+                } else {
+                    for (int cl = 0; cl < 2; cl++) {
+                        R v = tx[i] * M.R2[i][0][cl] + ty[i] * M.R2[i][1][cl];
+                        ksumr += v * v;
+                    }
                 }
+            }
+        };
+        layered_mb_rows<R, 3>(M, gc, lm, ln, sqrt(AeR), rows, rs, add);
+        R ws = stab * AeR * (R)(AVGK ? 1.0 / 3 : 1.0);
+        for (int o = 0; o < NS / 2; o++)
+            layered_shear_rows<R, 3>(M, gc, lm, ln, sqrt(ws), (const R(*)[3][5])sh[2 * o], rows + (6 + 2 * o) * rs, rs,
+                                     [&](int r, const R *tx, const R *ty) { add(6 + 2 * o + r, tx, ty); });
+        if constexpr (sizeof(R) == 4)
+            for (int i = 0; i < 3; i++)
+                for (int cl = 0; cl < 2; cl++)
+                    for (int r = 0; r < 6 + NS; r++) {
+                        R v = ltx[r][i] * M.R2[i][0][cl] + lty[r][i] * M.R2[i][1][cl];
+                        ksumr += v * v;
+                    }
         double kavg = drill_mean<R>((double)ksumr, mc);
         R sk = kavg > 0.0 ? sqrt((R)kavg) : (R)0;
         for (int i = 0; i < 3; i++) {
-            R *o = rows + (6 + NS + i) * rs;
-            for (int q = 0; q < 18; q++) o[q] = 0;
-            if (in.valid[i])
-                for (int c = 0; c < 3; c++) o[6 * i + 3 + c] = sk * M.t[i][2][c];
+            R *o = COMPACT ? rows + LayeredRows<3, 6 + NS>::DR + 3 * i : rows + (6 + NS + i) * rs;
+            if constexpr (!COMPACT)
+                for (int q = 0; q < 18; q++) o[q] = 0;
+            R *oc = COMPACT ? o : o + 6 * i + 3;
+            if (COMPACT || in.valid[i])
+                for (int c = 0; c < 3; c++) oc[c] = in.valid[i] ? sk * M.t[i][2][c] : (R)0;
         }
         return (kavg < 0.0) ? 2 : 0;
     }
@@ -954,27 +1034,11 @@ FS_HD int q4_point_rows(const ElemIn<4> &in, const Q4Elem &qe, int j, const MatC
                                   COMPACT ? rows + Q4Compact::BS + Q4Compact::BSS * (3 + r) : rows + (6 + r) * rs);
         }
     } else {
-        R mb[6][4][5];
-        for (int r = 0; r < 6; r++)
-            for (int i = 0; i < 4; i++)
-                for (int q = 0; q < 5; q++) mb[r][i][q] = 0;
-        for (int i = 0; i < 4; i++) {
-            mb[0][i][0] = g[i][0];
-            mb[1][i][1] = g[i][1];
-            mb[2][i][0] = g[i][1]; mb[2][i][1] = g[i][0];
-            mb[3][i][4] = g[i][0];
-            mb[4][i][3] = -g[i][1];
-            mb[5][i][3] = -g[i][0]; mb[5][i][4] = g[i][1];
-        }
-        R mixed[8][4][5];
         double lm, ln;
         layup_angle(e, gc->csmat, lm, ln);
-        rotate3<R, 4>(lm, ln, (R(*)[4][5])mb[0]);
-        rotate3<R, 4>(lm, ln, (R(*)[4][5])mb[3]);
-        mix_rows<R, 4, 6>(gc->L6, gc->L6f, sqrt(Jac), mb, (R(*)[4][5])mixed[0]);
-        rotate2<R, 4>(lm, ln, sh);
-        mix_rows<R, 4, 2>(gc->LH, gc->LHf, sqrt(stab * Jac), sh, (R(*)[4][5])mixed[6]);
-        for (int r = 0; r < 8; r++) expand_row<R, 4>(M, (const R(*)[5])mixed[r], rows + r * rs);
+        auto none = [](int, const R *, const R *) {};
+        layered_mb_rows<R, 4>(M, gc, lm, ln, sqrt(Jac), rows, rs, none);
+        layered_shear_rows<R, 4>(M, gc, lm, ln, sqrt(stab * Jac), sh, rows + 6 * rs, rs, none);
     }
     // drilling traces: sum over rows of |b|^2 - (b.n)^2 on the rotation block
     // (float rows: the float copy of the normals, the same values as the

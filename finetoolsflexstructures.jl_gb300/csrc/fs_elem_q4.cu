@@ -8,7 +8,8 @@
 // stabilisation factor, drilling factor) is split over the four lanes by
 // node where it is node-wise.  Homogeneous elements keep their rows in the
 // compact layout (Q4Compact: membrane rows on the translations, drilling rows
-// on one node's rotations), layered ones in the dense 36 x 24 layout.
+// on one node's rotations), layered ones as 32 dense rows and the drilling
+// rows (LayeredRows).
 #include "fs_elem_common.cuh"
 
 namespace fs {
@@ -21,7 +22,7 @@ struct Q4Stage {
 
 // row values (R units) one element keeps in shared memory, with one of
 // padding (an odd stride spreads the elements over the banks)
-__host__ __device__ constexpr int q4_row_values(bool layered) { return layered ? 36 * 24 + 1 : Q4Compact::SIZE + 1; }
+__host__ __device__ constexpr int q4_row_values(bool layered) { return (layered ? LayeredRows<4, 32>::SIZE : Q4Compact::SIZE) | 1; }
 
 size_t q4_smem(int precision, bool layered, int epb)
 {
@@ -41,6 +42,7 @@ __global__ void __launch_bounds__(128, 2)
     k_q4_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
     constexpr int ND = 24;
+    constexpr int DR = COMP ? LayeredRows<4, 32>::DR : Q4Compact::DR;
     constexpr int RV = q4_row_values(COMP);
     constexpr size_t RB = ((size_t)RV * sizeof(R) + 7) & ~(size_t)7;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -142,12 +144,8 @@ __global__ void __launch_bounds__(128, 2)
                 }
             const float kavg = (cnt ? sum / (float)cnt : 0.f) * (float)mc.drill_scale;
             const float sk = kavg > 0.f ? sqrtf(kavg) : 0.f;
-            R *o = rows + Q4Compact::DR + 3 * qp;
-            if constexpr (COMP) o = rows + (32 + qp) * ND;
-            if constexpr (COMP)
-                for (int q = 0; q < 24; q++) o[q] = 0;
-            R *oc = COMP ? o + 6 * qp + 3 : o;
-            for (int c = 0; c < 3; c++) oc[c] = (use && kavg != 0.f) ? (R)(sk * sg.in.nrmf[qp][c]) : (R)0;
+            R *o = rows + DR + 3 * qp;
+            for (int c = 0; c < 3; c++) o[c] = (use && kavg != 0.f) ? (R)(sk * sg.in.nrmf[qp][c]) : (R)0;
         }
     } else {
     // sum the drilling traces of the four quadrature points (lanes 4el..4el+3)
@@ -174,15 +172,8 @@ __global__ void __launch_bounds__(128, 2)
             }
         const double kavg = (cnt ? sum / cnt : 0.0) * mc.drill_scale;
         const double sk = kavg > 0.0 ? sqrt(kavg) : 0.0;
-        if constexpr (COMP) {
-            R *o = rows + (32 + qp) * ND;
-            for (int q = 0; q < 24; q++) o[q] = 0;
-            if (use && kavg != 0.0)
-                for (int c = 0; c < 3; c++) o[6 * qp + 3 + c] = (R)(sk * sg.in.nrm[qp][c]);
-        } else {
-            R *o = rows + Q4Compact::DR + 3 * qp;
-            for (int c = 0; c < 3; c++) o[c] = (use && kavg != 0.0) ? (R)(sk * sg.in.nrm[qp][c]) : (R)0;
-        }
+        R *o = rows + DR + 3 * qp;
+        for (int c = 0; c < 3; c++) o[c] = (use && kavg != 0.0) ? (R)(sk * sg.in.nrm[qp][c]) : (R)0;
     }
     }
     __syncwarp();
@@ -195,9 +186,8 @@ __global__ void __launch_bounds__(128, 2)
     // (its upper triangle), then the six off-diagonal blocks as twelve
     // half-blocks (rows 0-2 of each, then rows 3-5), three per lane.
     // Homogeneous elements: per Gauss point 3 membrane rows (translations
-    // only, so rows 0-2 of a block) and 5 bending/shear rows; then one
-    // drilling row per node (diagonal blocks only) -- the products and their
-    // order of the dense layout.
+    // only, so rows 0-2 of a block) and 5 bending/shear rows.  Layered ones: 32
+    // dense rows.  Then one drilling row per node (diagonal blocks only).
     {
         const int a = qp;
         BlockAcc<R, PAIR> acc;
@@ -209,10 +199,10 @@ __global__ void __launch_bounds__(128, 2)
                 gram_rows_c<0, 3, 0, 3, Q4Compact::MS, 3, 0, true>(acc, gpb, 0, 3, a, a);
                 gram_rows_c<0, 6, 0, 6, Q4Compact::BSS, 6, 0, true>(acc, gpb + Q4Compact::BS, 0, 5, a, a);
             }
-            gram_rows_c<3, 6, 3, 6, 3, 0, 3, true>(acc, rows + Q4Compact::DR + 3 * a, 0, 1, a, a);
         } else {
-            gram_rows<0, 6, 0, 6, true>(acc, rows, ND, 0, 36, a, a);
+            gram_rows_c<0, 6, 0, 6, ND, 6, 0, true>(acc, rows, 0, 32, a, a);
         }
+        gram_rows_c<3, 6, 3, 6, 3, 0, 3, true>(acc, rows + DR + 3 * a, 0, 1, a, a);
         acc.template store<true>(out + ub(a, a, 4) * 36);
     }
 #pragma unroll 1
@@ -234,7 +224,7 @@ __global__ void __launch_bounds__(128, 2)
                 gram_rows_h<0, 6, Q4Compact::BSS, 6>(acc, gpb + Q4Compact::BS, 0, 5, a, b, i0);
             }
         } else {
-            gram_rows_h<0, 6, ND, 6>(acc, rows, 0, 36, a, b, i0);
+            gram_rows_h<0, 6, ND, 6>(acc, rows, 0, 32, a, b, i0);
         }
         acc.store(out + ub(a0, b0, 4) * 36 + 6 * i0);
     }

@@ -24,12 +24,12 @@ template <class R, bool COMP, bool AVGK, class S>
 __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     k_t3_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
-    constexpr int NR = T3Rows<AVGK>::N, NS = T3Rows<AVGK>::NS;
+    constexpr int NS = T3Rows<AVGK>::NS;
     constexpr int ND = 18;
     // homogeneous elements: the compact rows (126 values instead of 198);
-    // layered ones: dense rows.  An odd stride keeps the threads' rows in
-    // distinct shared-memory banks.
-    constexpr int STRIDE = COMP ? NR * ND + 1 : CompactRows<3, NS>::SIZE + 1;
+    // layered ones: dense rows and the drilling rows' rotations (153).  An odd
+    // stride keeps the threads' rows in distinct shared-memory banks.
+    constexpr int STRIDE = (COMP ? LayeredRows<3, 6 + NS>::SIZE : CompactRows<3, NS>::SIZE) | 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *rows = reinterpret_cast<R *>(smem_raw) + threadIdx.x * STRIDE;
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -37,11 +37,11 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     ElemIn<3> in;
     load_elem<3>(m, r, in);
     const GroupConst *gc = COMP ? &m.groups[in.group] : nullptr;
-    int st = t3_rows<R, COMP, AVGK, !COMP>(in, mc, gc, rows, ND);
+    int st = t3_rows<R, COMP, AVGK, true>(in, mc, gc, rows, ND);
     if (st) atomicOr(status, DEV_NEG_DRILL);
     const unsigned swapped = swapped_blocks<3>(m.conn + r * 3);
     if constexpr (COMP)
-        write_blocks<R, S, 3, false>(rows, NR, swapped, ke + r * (6 * 36));
+        write_blocks_layered<R, S, 3, 6 + NS>(rows, swapped, ke + r * (6 * 36));
     else
         write_blocks_compact<R, S, 3, NS>(rows, swapped, ke + r * (6 * 36));
 }

@@ -28,9 +28,8 @@ namespace fs {
 // Shared memory of one block of the element kernels (per-element Gram rows).
 size_t t3_smem(int precision, bool avgk, bool layered, int epb)
 {
-    const int nr = avgk ? T3Rows<true>::N : T3Rows<false>::N;
-    const int per = layered ? nr * 18 + 1
-                            : (avgk ? CompactRows<3, T3Rows<true>::NS>::SIZE : CompactRows<3, T3Rows<false>::NS>::SIZE) + 1;
+    const int per = (layered ? (avgk ? LayeredRows<3, 6 + T3Rows<true>::NS>::SIZE : LayeredRows<3, 6 + T3Rows<false>::NS>::SIZE)
+                             : (avgk ? CompactRows<3, T3Rows<true>::NS>::SIZE : CompactRows<3, T3Rows<false>::NS>::SIZE)) | 1;
     return (precision == FS_FP64 ? 8 : 4) * (size_t)epb * per;
 }
 
