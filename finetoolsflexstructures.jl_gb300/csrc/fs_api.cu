@@ -499,7 +499,7 @@ int fs::assemble_matrix(fs_ctx *c, int precision, int assembler, int64_t nrows, 
     c->mat_colidx = P.colidx;
     c->mat_nnz = P.nnz;
     if (assembler == FS_ASM_SPARSE_SYMM) {
-        FS_TRY(compact_zeros(c, nrows, P.rowptr, P.colidx, c->vals, P.nnz));
+        FS_TRY(compact_zeros(c, nrows, P.rowptr, P.colidx, P.nnz));
         FS_CUDA(c, cudaEventRecord(c->ev[3], c->stream));
         FS_CUDA(c, cudaEventSynchronize(c->ev[3]));
         float ms = 0.f;

@@ -160,7 +160,7 @@ struct fs_ctx {
     int64_t *cmp_rowptr = nullptr;
     int32_t *cmp_colidx = nullptr;
     double *cmp_vals = nullptr;
-    size_t cmp_cap = 0;
+    size_t cap_cmp_rowptr = 0, cap_cmp_colidx = 0, cmp_vals_cap = 0;
     // phase timing events: element start/end, gather end, compaction end
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     double t_symbolic_ms = 0.0;
@@ -262,8 +262,7 @@ int launch_elements_to(fs_ctx *c, int precision, void *ke);
 int launch_gather_from(fs_ctx *c, int precision, const void *ke, double *vals);
 int launch_masses(fs_ctx *c);
 int assemble_mass(fs_ctx *c, int assembler, int64_t n);
-int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *colidx,
-                  const double *vals, int64_t nnz);
+int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *colidx, int64_t nnz);
 int exclusive_scan_i64(fs_ctx *c, const int64_t *in, int64_t *out, int64_t n, int64_t *total);
 int ensure_scratch(fs_ctx *c, size_t bytes);
 int read_status(fs_ctx *c, int *bits);

@@ -604,39 +604,59 @@ int build_pattern(fs_ctx *c, int64_t n)
 // dropping exact zeros (FinEtools SysmatAssemblerSparseSymm: S + S^T keeps
 // only nonzero results)
 // ---------------------------------------------------------------------------
-__global__ void k_count_nonzero(int64_t n, const int64_t *rowptr, const double *vals, int64_t *cnt)
+// 16 lanes a row, so that a warp reads whole lines and has loads enough in
+// flight: both kernels run at the memory's pace (one thread a row, a copy back
+// and buffers allocated for each call: triangles, 700 x 700, 9.5 ms; now 1.0).
+static const int ROW_LANES = 16;
+
+__global__ void k_count_nonzero(int64_t n, const int64_t *__restrict__ rowptr, const double *__restrict__ vals, int64_t *cnt)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int64_t s = 0;
-    for (int64_t k = rowptr[i]; k < rowptr[i + 1]; k++) s += (vals[k] != 0.0);
-    cnt[i] = s;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / ROW_LANES;
+    int s = 0;
+    if (i < n) {
+        const int64_t e = rowptr[i + 1];
+#pragma unroll 4
+        for (int64_t k = rowptr[i] + threadIdx.x % ROW_LANES; k < e; k += ROW_LANES) s += vals[k] != 0.0;
+    }
+#pragma unroll
+    for (int o = ROW_LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (i < n && threadIdx.x % ROW_LANES == 0) cnt[i] = s;
 }
 
-__global__ void k_compact(int64_t n, const int64_t *rowptr, const int32_t *colidx, const double *vals,
-                          const int64_t *nrowptr, int32_t *ncol, double *nval)
+__global__ void k_compact(int64_t n, const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
+                          const double *__restrict__ vals, const int64_t *__restrict__ nrowptr, int32_t *__restrict__ ncol,
+                          double *__restrict__ nval)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / ROW_LANES;
     if (i >= n) return;
+    const int sub = threadIdx.x % ROW_LANES, shift = (threadIdx.x & 31) - sub;
+    const unsigned row = ((1u << ROW_LANES) - 1) << shift;   // this row's lanes
+    const int64_t e = rowptr[i + 1];
     int64_t w = nrowptr[i];
-    for (int64_t k = rowptr[i]; k < rowptr[i + 1]; k++)
-        if (vals[k] != 0.0) {
-            ncol[w] = colidx[k];
-            nval[w] = vals[k];
-            w++;
+#pragma unroll 4
+    for (int64_t k = rowptr[i] + sub; k - sub < e; k += ROW_LANES) {
+        const double v = k < e ? vals[k] : 0.0;
+        const int32_t c = k < e ? colidx[k] : 0;
+        const unsigned keep = __ballot_sync(row, v != 0.0) >> shift;
+        if (v != 0.0) {
+            const int64_t at = w + __popc(keep & ((1u << sub) - 1));
+            ncol[at] = c;
+            nval[at] = v;
         }
+        w += __popc(keep);
+    }
 }
 
-int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *colidx, const double *vals,
-                  int64_t nnz)
+// The matrix without its exact zeros: the kept entries go to a second pair of
+// buffers, and the two value buffers change places
+int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *colidx, int64_t nnz)
 {
-    int64_t *cnt = nullptr;
-    FS_TRY(dalloc(c, &cnt, (size_t)n));
-    if (n) k_count_nonzero<<<nblk(n, 256), 256, 0, c->stream>>>(n, rowptr, vals, cnt);
-    FS_TRY(dalloc(c, &c->cmp_rowptr, (size_t)n + 1));
+    FS_TRY(grow(c, &c->pat.tmp_cnt, &c->pat.cap_tmp_cnt, (size_t)n));
+    FS_TRY(grow(c, &c->cmp_rowptr, &c->cap_cmp_rowptr, (size_t)n + 1));
+    int64_t *cnt = c->pat.tmp_cnt;
+    if (n) k_count_nonzero<<<nblk(n * ROW_LANES, 256), 256, 0, c->stream>>>(n, rowptr, c->vals, cnt);
     int64_t nnz2 = 0;
     FS_TRY(exclusive_scan_i64(c, cnt, c->cmp_rowptr, n, &nnz2));
-    cudaFree(cnt);
     if (nnz2 == nnz) {
         // nothing to drop: keep the arrays as they are
         c->mat_rowptr = rowptr;
@@ -644,14 +664,18 @@ int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *co
         c->mat_nnz = nnz;
         return FS_OK;
     }
-    if ((size_t)nnz2 > c->cmp_cap || !c->cmp_colidx) {
-        FS_TRY(dalloc(c, &c->cmp_colidx, (size_t)nnz2));
-        FS_TRY(dalloc(c, &c->cmp_vals, (size_t)nnz2));
-        c->cmp_cap = (size_t)nnz2;
-    }
-    if (n) k_compact<<<nblk(n, 256), 256, 0, c->stream>>>(n, rowptr, colidx, vals, c->cmp_rowptr, c->cmp_colidx, c->cmp_vals);
+    FS_TRY(grow(c, &c->cmp_colidx, &c->cap_cmp_colidx, (size_t)nnz2));
+    // as large as the first buffer, so that the next assembly can use it; where
+    // there is no memory for that, as large as it must be, and copied back
+    if (c->cmp_vals_cap < c->vals_cap && grow(c, &c->cmp_vals, &c->cmp_vals_cap, c->vals_cap) != FS_OK)
+        FS_TRY(grow(c, &c->cmp_vals, &c->cmp_vals_cap, (size_t)nnz2));
+    if (n) k_compact<<<nblk(n * ROW_LANES, 256), 256, 0, c->stream>>>(n, rowptr, colidx, c->vals, c->cmp_rowptr, c->cmp_colidx, c->cmp_vals);
     FS_CUDA(c, cudaGetLastError());
-    FS_CUDA(c, cudaMemcpyAsync(c->vals, c->cmp_vals, sizeof(double) * nnz2, cudaMemcpyDeviceToDevice, c->stream));
+    if (c->cmp_vals_cap >= c->vals_cap) {
+        std::swap(c->vals, c->cmp_vals);
+        std::swap(c->vals_cap, c->cmp_vals_cap);
+    } else
+        FS_CUDA(c, cudaMemcpyAsync(c->vals, c->cmp_vals, sizeof(double) * nnz2, cudaMemcpyDeviceToDevice, c->stream));
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->mat_rowptr = c->cmp_rowptr;
     c->mat_colidx = c->cmp_colidx;
