@@ -84,6 +84,11 @@ __global__ void k_fill_d(int64_t n, double v, double *p)
     if (i < n) p[i] = v;
 }
 
+__global__ void k_to_i32(int64_t n, const int64_t *src, int32_t *dst)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = (int32_t)src[i];
+}
 __global__ void k_plus_one_i64(int64_t n, const int64_t *src, int64_t *dst)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -620,6 +625,25 @@ int fs_matrix_copy(fs_ctx *c, int64_t *colptr, int64_t *rowval, double *nzval)
         FS_CUDA(c, cudaMemcpyAsync(rowval, c->stage64, sizeof(int64_t) * nnz, cudaMemcpyDeviceToHost, c->stream));
     }
     if (nzval && nnz) FS_CUDA(c, cudaMemcpyAsync(nzval, c->vals, sizeof(double) * nnz, cudaMemcpyDeviceToHost, c->stream));
+    FS_CUDA(c, cudaStreamSynchronize(c->stream));
+    return FS_OK;
+}
+
+int fs_matrix_copy_i32(fs_ctx *c, int32_t *colptr, int32_t *rowval, double *nzval)
+{
+    if (!c) return FS_ERR_BAD_INPUT;
+    FS_CUDA(c, cudaSetDevice(c->device));
+    if (!c->mat_rowptr) return set_err(c, FS_ERR_STATE, "no matrix assembled");
+    const int64_t n = c->mat_n, nnz = c->mat_nnz;
+    if (nnz > 0x7fffffffLL) return set_err(c, FS_ERR_UNSUPPORTED, "more entries than 32-bit indices can count");
+    if (colptr) {
+        FS_TRY(ensure_scratch(c, sizeof(int32_t) * (size_t)(n + 1)));
+        k_to_i32<<<(unsigned)((n + 1 + 255) / 256), 256, 0, c->stream>>>(n + 1, c->mat_rowptr, (int32_t *)c->scratch);
+        FS_CUDA(c, cudaGetLastError());
+        FS_CUDA(c, cudaMemcpyAsync(colptr, c->scratch, sizeof(int32_t) * (size_t)(n + 1), cudaMemcpyDeviceToHost, c->stream));
+    }
+    if (rowval && nnz) FS_CUDA(c, cudaMemcpyAsync(rowval, c->mat_colidx, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream));
+    if (nzval && nnz) FS_CUDA(c, cudaMemcpyAsync(nzval, c->vals, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream));
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     return FS_OK;
 }

@@ -46,6 +46,7 @@ def lib():
         L.fs_stiffness.argtypes = [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int64, _c_i64_p]
         L.fs_mass.argtypes = [vp, ctypes.c_int, ctypes.c_int64, _c_i64_p]
         L.fs_matrix_copy.argtypes = [vp, vp, vp, vp]
+        L.fs_matrix_copy_i32.argtypes = [vp, vp, vp, vp]
         L.fs_matrix_device.argtypes = [vp, ctypes.POINTER(vp), ctypes.POINTER(vp), ctypes.POINTER(vp),
                                        _c_i64_p, _c_i64_p]
         L.fs_element_matrices.argtypes = [vp, ctypes.c_int, vp]
@@ -136,6 +137,21 @@ class Context:
 
     def call(self, name, *args):
         self.check(getattr(lib(), name)(self._h, *args))
+
+    def matrix(self, nrows, nnz):
+        """The last matrix as (values, indices, indptr), 0-based; 32-bit indices
+        where they can count the entries, which is how scipy keeps them (64-bit ones
+        it searches and converts: quads, 120 x 75, a model's two matrices in
+        6.4 ms, now 1.4)."""
+        nzval = np.empty(nnz, dtype=np.float64)
+        small = nnz < 1 << 31
+        colptr = np.empty(nrows + 1, dtype=np.int32 if small else np.int64)
+        rowval = np.empty(nnz, dtype=colptr.dtype)
+        self.call("fs_matrix_copy_i32" if small else "fs_matrix_copy", ptr(colptr), ptr(rowval), ptr(nzval))
+        if not small:
+            colptr -= 1
+            rowval -= 1
+        return nzval, rowval, colptr
 
     def stream(self):
         s = ctypes.c_void_p()

@@ -322,12 +322,8 @@ class FEMMCorotBeam:
         nrows = assembler.nrows if assembler.nrows is not None else dchi.nalldofs()
         nnz = ctypes.c_int64()
         self.ctx.call("fs_beam_matrix", which, mass_type, assembler.mode, nrows, ctypes.byref(nnz))
-        colptr = np.empty(nrows + 1, dtype=np.int64)
-        rowval = np.empty(nnz.value, dtype=np.int64)
-        nzval = np.empty(nnz.value, dtype=np.float64)
-        self.ctx.call("fs_matrix_copy", ptr(colptr), ptr(rowval), ptr(nzval))
         cls = sp.csr_matrix if assembler.csr else sp.csc_matrix
-        return cls((nzval, rowval - 1, colptr - 1), shape=(nrows, nrows))
+        return cls(self.ctx.matrix(nrows, nnz.value), shape=(nrows, nrows))
 
     @staticmethod
     def _split(args, n):

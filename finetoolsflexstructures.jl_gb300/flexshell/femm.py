@@ -244,13 +244,8 @@ class _FEMMShell:
 
     def _fetch(self, nrows, nnz, csr):
         import scipy.sparse as sp
-        colptr = np.empty(nrows + 1, dtype=np.int64)
-        rowval = np.empty(nnz, dtype=np.int64)
-        nzval = np.empty(nnz, dtype=np.float64)
-        self.ctx.call("fs_matrix_copy", ptr(colptr), ptr(rowval), ptr(nzval))
-        if csr:
-            return sp.csr_matrix((nzval, rowval - 1, colptr - 1), shape=(nrows, nrows))
-        return sp.csc_matrix((nzval, rowval - 1, colptr - 1), shape=(nrows, nrows))
+        cls = sp.csr_matrix if csr else sp.csc_matrix
+        return cls(self.ctx.matrix(nrows, nnz), shape=(nrows, nrows))
 
     def stiffness(self, assembler, geom0, u1=None, Rfield1=None, dchi=None, precision=FS_FP64):
         """stiffness(femm, assembler, geom0, u1, Rfield1, dchi) -> K."""

@@ -162,6 +162,9 @@ int fs_mass(fs_ctx *ctx, int assembler, int64_t nrows, int64_t *nnz_out);
 /* The matrix of the last fs_stiffness / fs_mass call into caller memory:
  * colptr[nrows+1], rowval[nnz], nzval[nnz], 1-based CSC.  Any pointer may be NULL. */
 int fs_matrix_copy(fs_ctx *ctx, int64_t *colptr, int64_t *rowval, double *nzval);
+/* The same with 0-based 32-bit indices, as scipy keeps them (half the bytes and
+ * no conversion on the host); FS_ERR_UNSUPPORTED for 2^31 entries or more. */
+int fs_matrix_copy_i32(fs_ctx *ctx, int32_t *colptr, int32_t *rowval, double *nzval);
 /* Two-phase stiffness into host arrays for the pattern-keeping assembler
  * (FS_ASM_SPARSE, also the FF block with nrows = nfreedofs): fs_pattern builds
  * (or reuses) the pattern for `nrows` and returns the number of stored entries,
