@@ -13,7 +13,7 @@
 #include <cmath>
 #include <cstring>
 
-#include "fs_internal.cuh"
+#include "fs_elem_common.cuh"
 
 static_assert(sizeof(fs_beam_section) == sizeof(fs::BeamSection), "section layouts differ");
 
@@ -45,13 +45,6 @@ __device__ __forceinline__ void beam_load(const MeshDev &m, const BeamDev &b, in
             for (int j = 0; j < 3; j++)
                 R[a][i][j] = b.R1 ? b.R1[(int64_t)(i + 3 * j) * m.nnodes + node] : (i == j ? 1.0 : 0.0);
     }
-}
-
-__device__ __forceinline__ void store_block_d(double *o, const double (&acc)[6][6])
-{
-    double2 *o2 = reinterpret_cast<double2 *>(o);
-#pragma unroll
-    for (int q = 0; q < 18; q++) o2[q] = make_double2(acc[(2 * q) / 6][(2 * q) % 6], acc[(2 * q + 1) / 6][(2 * q + 1) % 6]);
 }
 
 __device__ __forceinline__ void beam_prepare_rank(const MeshDev &m, const BeamDev &b, int64_t r, bool velocities,
@@ -92,7 +85,7 @@ __global__ void __launch_bounds__(128) k_beam_elements(const MeshDev m, const Be
                         acc[j][i] = t;
                     }
             }
-            store_block_d(out + ub(a, bb, 2) * 36, acc);
+            store_rows<double, 6>(out + ub(a, bb, 2) * 36, acc);
         }
 }
 

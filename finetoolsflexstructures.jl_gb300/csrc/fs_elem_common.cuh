@@ -26,38 +26,58 @@ __device__ __forceinline__ void load_elem(const MeshDev &m, int64_t r, ElemIn<NN
     in.group = m.group ? m.group[r] : 0;
 }
 
+// P 16-byte pieces to a 16-byte boundary (32 bytes for an even P), in 32-byte
+// stores: a thread writes its own stretch of memory, so a store instruction
+// touches 32 lines, and two 16-byte stores to a sector also cost the L2 a write
+// each (triangles, 1024 x 1024, FS_MIXED_COMP: 1.25 ms, now 1.00)
+__device__ __forceinline__ void store_16(void *p, const uint32_t *w)
+{
+    *reinterpret_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void store_32(void *p, const uint32_t *w)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(__cvta_generic_to_global(p)), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+template <int P> __device__ __forceinline__ void store_pieces(void *p, const uint32_t (&w)[4 * P])
+{
+    char *o = reinterpret_cast<char *>(p);
+    if ((P & 1) && (reinterpret_cast<uintptr_t>(p) & 16)) {
+        store_16(o, w);
+#pragma unroll
+        for (int q = 1; q + 1 < P; q += 2) store_32(o + 16 * q, w + 4 * q);
+    } else {
+#pragma unroll
+        for (int q = 0; q + 1 < P; q += 2) store_32(o + 16 * q, w + 4 * q);
+        if (P & 1) store_16(o + 16 * (P - 1), w + 4 * (P - 1));
+    }
+}
+
 // NI rows of a 6x6 block (6 NI contiguous values from a 16-byte boundary for
-// whole blocks, an 8-byte one for the half-blocks of float values): 16-byte
-// stores, or 8-byte ones for float half-blocks
+// whole blocks, an 8-byte one for the half-blocks of float values): 8-byte
+// stores for float half-blocks
 template <class R, int NI>
 __device__ __forceinline__ void store_rows(R *o, const R (&acc)[NI][6])
 {
     if (sizeof(R) == 4 && NI == 6) {
-        float4 *o4 = reinterpret_cast<float4 *>(o);
+        uint32_t w[36];
 #pragma unroll
-        for (int q = 0; q < 9; q++) {
-            const int e = 4 * q;
-            o4[q] = make_float4((float)acc[e / 6][e % 6], (float)acc[(e + 1) / 6][(e + 1) % 6],
-                                (float)acc[(e + 2) / 6][(e + 2) % 6], (float)acc[(e + 3) / 6][(e + 3) % 6]);
-        }
+        for (int e = 0; e < 36; e++) w[e] = __float_as_uint((float)acc[e / 6 % NI][e % 6]);
+        store_pieces<9>(o, w);
     } else if (sizeof(R) == 4) {
         float2 *o2 = reinterpret_cast<float2 *>(o);
 #pragma unroll
         for (int q = 0; q < 3 * NI; q++) o2[q] = make_float2((float)acc[q / 3][2 * (q % 3)], (float)acc[q / 3][2 * (q % 3) + 1]);
     } else {
-        double2 *o2 = reinterpret_cast<double2 *>(o);
+        uint32_t w[12 * NI];
 #pragma unroll
-        for (int q = 0; q < 3 * NI; q++)
-            o2[q] = make_double2((double)acc[q / 3][2 * (q % 3)], (double)acc[q / 3][2 * (q % 3) + 1]);
+        for (int e = 0; e < 6 * NI; e++) {
+            w[2 * e] = (uint32_t)__double2loint((double)acc[e / 6][e % 6]);
+            w[2 * e + 1] = (uint32_t)__double2hiint((double)acc[e / 6][e % 6]);
+        }
+        store_pieces<3 * NI>(o, w);
     }
-}
-
-// three rows of a 6x6 block of doubles (16-byte stores)
-__device__ __forceinline__ void store_half(double *o, const double (&v)[3][6])
-{
-    double2 *o2 = reinterpret_cast<double2 *>(o);
-#pragma unroll
-    for (int q = 0; q < 9; q++) o2[q] = make_double2(v[q / 3][2 * (q % 3)], v[q / 3][2 * (q % 3) + 1]);
 }
 
 // One step of a compensated dot product (Ogita, Rump and Oishi's Dot2):
@@ -173,12 +193,17 @@ template <int NI, int LEVELS = 3> struct PairAcc {
                     l[i][j] = l[j][i];
                 }
         }
-        float4 *o4 = reinterpret_cast<float4 *>(o);
+        uint32_t w[12 * NI];
 #pragma unroll
         for (int i = 0; i < NI; i++)
 #pragma unroll
-            for (int q = 0; q < 3; q++)
-                o4[3 * i + q] = make_float4(h[i][2 * q], h[i][2 * q + 1], l[i][2 * q], l[i][2 * q + 1]);
+            for (int q = 0; q < 3; q++) {
+                w[12 * i + 4 * q] = __float_as_uint(h[i][2 * q]);
+                w[12 * i + 4 * q + 1] = __float_as_uint(h[i][2 * q + 1]);
+                w[12 * i + 4 * q + 2] = __float_as_uint(l[i][2 * q]);
+                w[12 * i + 4 * q + 3] = __float_as_uint(l[i][2 * q + 1]);
+            }
+        store_pieces<3 * NI>(o, w);
     }
 };
 template <int NI> struct BlockAcc<float, true, NI> : PairAcc<NI, Q4_PAIR_LEVELS> {};

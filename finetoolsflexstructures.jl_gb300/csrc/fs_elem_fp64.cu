@@ -104,13 +104,13 @@ __global__ void __launch_bounds__(96, 4) k_t3_gram(const MeshDev m, int64_t e0, 
     {
         double o[3][6], ob[3][6];
         fx_block_top<1, L::MS, L::BS, L::BSS, true>(slot, 0, w, w, ex, o);
-        store_half(out + ub(w, w, 3) * 36, o);
+        store_rows<double, 3>(out + ub(w, w, 3) * 36, o);
         fx_block_bottom<1, L::BS, L::BSS, true>(slot, 0, w, w, slot + (L::DR + 3 * w), ex, ob);
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = 0; j < 3; j++) ob[i][j] = o[j][3 + i];
-        store_half(out + ub(w, w, 3) * 36 + 18, ob);
+        store_rows<double, 3>(out + ub(w, w, 3) * 36 + 18, ob);
     }
     // blocks (0,1) (0,2) (1,2), the lower node's dofs as rows
     const int a = w == 2 ? 1 : 0, b = w == 0 ? 1 : 2;
@@ -118,9 +118,9 @@ __global__ void __launch_bounds__(96, 4) k_t3_gram(const MeshDev m, int64_t e0, 
     const int p = sw ? b : a, q = sw ? a : b;
     double o[3][6];
     fx_block_top<1, L::MS, L::BS, L::BSS, false>(slot, 0, p, q, ex, o);
-    store_half(out + ub(a, b, 3) * 36, o);
+    store_rows<double, 3>(out + ub(a, b, 3) * 36, o);
     fx_block_bottom<1, L::BS, L::BSS, false>(slot, 0, p, q, slot, ex, o);
-    store_half(out + ub(a, b, 3) * 36 + 18, o);
+    store_rows<double, 3>(out + ub(a, b, 3) * 36 + 18, o);
 }
 
 // per-element staging area of the Q4 rows kernel
@@ -246,13 +246,13 @@ __global__ void __launch_bounds__(128, 3) k_q4_gram(const MeshDev m, int64_t e0,
     {
         double o[3][6], ob[3][6];
         fx_block_top<4, L::MS, L::BS, L::BSS, true>(slot, L::GP, w, w, ex, o);
-        store_half(out + ub(w, w, 4) * 36, o);
+        store_rows<double, 3>(out + ub(w, w, 4) * 36, o);
         fx_block_bottom<4, L::BS, L::BSS, true>(slot, L::GP, w, w, slot + (L::DR + 3 * w), ex, ob);
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = 0; j < 3; j++) ob[i][j] = o[j][3 + i];
-        store_half(out + ub(w, w, 4) * 36 + 18, ob);
+        store_rows<double, 3>(out + ub(w, w, 4) * 36 + 18, ob);
     }
 #pragma unroll 1
     for (int t = 0; t < 3; t++) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(128, 3) k_q4_gram(const MeshDev m, int64_t e0,
             fx_block_top<4, L::MS, L::BS, L::BSS, false>(slot, L::GP, p, q, ex, o);
         else
             fx_block_bottom<4, L::BS, L::BSS, false>(slot, L::GP, p, q, slot, ex, o);
-        store_half(out + ub(a, b, 4) * 36 + (u < 6 ? 0 : 18), o);
+        store_rows<double, 3>(out + ub(a, b, 4) * 36 + (u < 6 ? 0 : 18), o);
     }
 }
 
