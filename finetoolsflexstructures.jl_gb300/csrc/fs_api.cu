@@ -223,7 +223,6 @@ int fs_ctx_destroy(fs_ctx *c)
     free_shift(c);
     if (c->ke) cudaFree(c->ke);
     if (c->fx_rows) cudaFree(c->fx_rows);
-    dfree(&c->fx_redo);
     dfree(&c->tmrm); dfree(&c->vals); dfree(&c->cmp_rowptr); dfree(&c->cmp_colidx); dfree(&c->cmp_vals);
     dfree(&c->stage64);
     if (c->scratch) cudaFree(c->scratch);

@@ -278,20 +278,22 @@ static int64_t chunk_elements(const MeshDev &m)
     return std::max<int64_t>((groups + chunks - 1) / chunks, 1) * FX_GROUP;
 }
 
-// The row buffer (one chunk) and the marks of the context's mesh, kept by the
-// context.  Where the memory for a whole chunk is not there, half of it is
-// tried, and so on; with no memory for the smallest, fx_rows stays null.
+// slots that the marks of the elements to do in double take, ahead of the rows
+static size_t mark_slots(const MeshDev &m) { return ((size_t)m.nelem + 255) / 256 * (256 / sizeof(FxSlot)); }
+
+// The buffer of the marks and of a chunk's rows, kept by the context.  Where the
+// memory for a whole chunk is not there, half of it is tried, and so on; with no
+// memory for the smallest, fx_rows stays null.
 int ensure_fp64_rows(fs_ctx *c)
 {
     const MeshDev &m = c->mesh;
     if (m.etype != FS_T3FF && m.etype != FS_Q4RS) return FS_OK;
-    FS_TRY(grow(c, &c->fx_redo, &c->cap_fx_redo, (size_t)m.nelem));
-    const size_t group = (size_t)FX_GROUP * (m.nen == 3 ? T3_SLOTS : Q4_SLOTS);
+    const size_t group = (size_t)FX_GROUP * (m.nen == 3 ? T3_SLOTS : Q4_SLOTS), marks = mark_slots(m);
     size_t want = (size_t)chunk_elements(m) / FX_GROUP;
-    if (c->fx_rows && c->fx_asked >= want * group) return FS_OK;
-    c->fx_asked = want * group;
+    if (c->fx_rows && c->fx_asked >= marks + want * group) return FS_OK;
+    c->fx_asked = marks + want * group;
     for (FxSlot *rows = (FxSlot *)c->fx_rows;; want /= 2) {
-        const int st = grow(c, &rows, &c->cap_fx_rows, want * group);
+        const int st = grow(c, &rows, &c->cap_fx_rows, marks + want * group);
         c->fx_rows = rows;
         if (st != FS_ERR_OOM) return st;
         if (want <= (size_t)FX_LEAST_GROUPS) return FS_OK;
@@ -304,8 +306,10 @@ int run_fp64(fs_ctx *c, double *ke)
     const bool t3 = m.nen == 3;
     FS_TRY(ensure_fp64_rows(c));
     if (!c->fx_rows) return t3 ? redo_t3(c, ke, nullptr) : redo_q4(c, ke, nullptr);
-    FxSlot *rows = (FxSlot *)c->fx_rows;
-    const int64_t fit = (int64_t)(c->cap_fx_rows / ((size_t)FX_GROUP * (t3 ? T3_SLOTS : Q4_SLOTS))) * FX_GROUP;
+    const size_t marks = mark_slots(m);
+    uint8_t *redo = (uint8_t *)c->fx_rows;
+    FxSlot *rows = (FxSlot *)c->fx_rows + marks;
+    const int64_t fit = (int64_t)((c->cap_fx_rows - marks) / ((size_t)FX_GROUP * (t3 ? T3_SLOTS : Q4_SLOTS))) * FX_GROUP;
     const int64_t chunk = std::min(chunk_elements(m), fit);
     int epb = c->tune.elem_epb;
     if (t3 && epb != 32 && epb != 64) epb = 128;
@@ -314,10 +318,10 @@ int run_fp64(fs_ctx *c, double *ke)
         const int64_t n = std::min(chunk, m.nelem - e0);
         const unsigned groups = (unsigned)((n + FX_GROUP - 1) / FX_GROUP);
         if (t3) {
-            k_t3_rows<<<nblk2(n, epb), epb, 0, c->stream>>>(m, c->mc, e0, n, rows, c->fx_redo, c->d_status);
+            k_t3_rows<<<nblk2(n, epb), epb, 0, c->stream>>>(m, c->mc, e0, n, rows, redo, c->d_status);
             k_t3_gram<<<groups, 96, sizeof(FxSlot) * FX_GROUP * T3_SLOTS, c->stream>>>(m, e0, n, rows, ke);
         } else {
-            k_q4_rows<<<nblk2(n, epb), 4 * epb, 0, c->stream>>>(m, c->mc, e0, n, rows, c->fx_redo, c->d_status);
+            k_q4_rows<<<nblk2(n, epb), 4 * epb, 0, c->stream>>>(m, c->mc, e0, n, rows, redo, c->d_status);
             k_q4_gram<<<groups, 128, 0, c->stream>>>(m, e0, n, rows, ke);
         }
     }
@@ -333,7 +337,7 @@ int read_element_status(fs_ctx *c, int precision, void *ke, double *vals, int *b
     FS_TRY(read_status(c, bits));
     if (!(*bits & DEV_REDO)) return FS_OK;
     const int first = *bits & ~DEV_REDO;
-    FS_TRY(c->mesh.nen == 3 ? redo_t3(c, (double *)ke, c->fx_redo) : redo_q4(c, (double *)ke, c->fx_redo));
+    FS_TRY(c->mesh.nen == 3 ? redo_t3(c, (double *)ke, (const uint8_t *)c->fx_rows) : redo_q4(c, (double *)ke, (const uint8_t *)c->fx_rows));
     if (vals) FS_TRY(launch_gather_from(c, precision, ke, vals));
     FS_TRY(read_status(c, bits));
     *bits |= first;

@@ -146,8 +146,6 @@ struct fs_ctx {
     void *fx_rows = nullptr;
     size_t cap_fx_rows = 0, fx_asked = 0;
     bool drops_zeros = false;  // during an assembly that drops exact zeros
-    uint8_t *fx_redo = nullptr;
-    size_t cap_fx_redo = 0;
     // current matrix; mat_kind 0 a stiffness (shell or beam), 1 a mass, 2
     // another beam matrix
     int mat_kind = -1;
