@@ -61,13 +61,13 @@ def params(quads):
 # under profiles/); the figures are scaled to the benchmark's element count,
 # traffic growing in proportion to the elements at a fixed mesh type.
 MEASURED_TRAFFIC_PER_ELEMENT = {
-    "k_t3_elements FS_MIXED": (802.2, "ncu --set full, k_t3_elements, FS_MIXED, T3FF 512^2 "
+    "k_t3_elements FS_MIXED": (797.6, "ncu --set full, k_t3_elements, FS_MIXED, T3FF 512^2 "
                                       "(profiles/k_t3_elements_k_gather_t3ff_mixed_512.md)"),
-    "k_gather FS_MIXED": (1983.5, "ncu --set full, k_gather, FS_MIXED, T3FF 512^2 "
+    "k_gather FS_MIXED": (1955.2, "ncu --set full, k_gather, FS_MIXED, T3FF 512^2 "
                                   "(profiles/k_t3_elements_k_gather_t3ff_mixed_512.md)"),
-    "k_t3_elements FS_MIXED_COMP": (1668.8, "ncu --set full, k_t3_elements, FS_MIXED_COMP, T3FF 512^2 "
+    "k_t3_elements FS_MIXED_COMP": (1661.4, "ncu --set full, k_t3_elements, FS_MIXED_COMP, T3FF 512^2 "
                                             "(profiles/k_t3_elements_k_gather_t3ff_mixed_comp_512.md)"),
-    "k_gather FS_MIXED_COMP": (2874.2, "ncu --set full, k_gather, FS_MIXED_COMP, T3FF 512^2 "
+    "k_gather FS_MIXED_COMP": (2838.5, "ncu --set full, k_gather, FS_MIXED_COMP, T3FF 512^2 "
                                        "(profiles/k_t3_elements_k_gather_t3ff_mixed_comp_512.md)"),
 }
 
@@ -374,7 +374,10 @@ def explicit_c5(torch, device=0, n=512, nsteps=10000, iters=200):
     rows_ = np.repeat(np.arange(conn.shape[0]), conn.shape[1])
     inc = sps.csr_matrix((np.ones(rows_.size), (rows_, conn.ravel() - 1)), shape=(conn.shape[0], nn_))
     nblocks = int((inc.T @ inc).nnz)
-    bsr_bytes = lambda es: nblocks * (36 * es + 4) + nn_ * (8 + 6 * 4) + nfree * (13 * 8 + 4 + es)
+    # each off-diagonal block once, an 8-byte item per block of a row, 12 passes
+    # over the state's vectors, the displacement copies (xs bytes a dof) read and written
+    bsr_bytes = lambda es, xs: ((nblocks + nn_) // 2 * 36 * es + nblocks * 8 + nn_ * (8 + 6 * 4) +
+                                nfree * 12 * 8 + 2 * 6 * nn_ * xs)
     out.update({"elements": conn.shape[0], "dofs": nfree, "nnz": nnz.value, "steps": nsteps,
                 "omega_max": om.value, "dt": dt, "power_iterations": iters,
                 "final_u_rel_err_mixed_vs_fp64": float(np.abs(U32 - U64).max() / np.abs(U64).max()),
@@ -383,11 +386,11 @@ def explicit_c5(torch, device=0, n=512, nsteps=10000, iters=200):
                               "float sum of K U",
                 "final_u_max": float(np.abs(U64).max()),
                 "format": "6x6 node blocks (block rows = node neighbour lists)", "blocks": nblocks,
-                "bytes_per_step_mixed": bsr_bytes(4), "bytes_per_step_fp64": bsr_bytes(8),
-                "hbm_gbs_mixed": bsr_bytes(4) * out["steps_per_s_mixed"] / 1e9,
-                "bytes_per_step_mixed_comp": bsr_bytes(6) + 6 * nn_ * 2,
-                "hbm_gbs_mixed_comp": (bsr_bytes(6) + 6 * nn_ * 2) * out["steps_per_s_mixed_comp"] / 1e9,
-                "hbm_gbs_fp64": bsr_bytes(8) * out["steps_per_s_fp64"] / 1e9})
+                "bytes_per_step_mixed": bsr_bytes(4, 4), "bytes_per_step_fp64": bsr_bytes(8, 8),
+                "hbm_gbs_mixed": bsr_bytes(4, 4) * out["steps_per_s_mixed"] / 1e9,
+                "bytes_per_step_mixed_comp": bsr_bytes(6, 8),
+                "hbm_gbs_mixed_comp": bsr_bytes(6, 8) * out["steps_per_s_mixed_comp"] / 1e9,
+                "hbm_gbs_fp64": bsr_bytes(8, 8) * out["steps_per_s_fp64"] / 1e9})
     ctx.close()
     return out
 
@@ -663,16 +666,16 @@ def t3_bytes(nelem, nnz, nodes, precision, pairs_once):
     entry for FS_MIXED, 8 for a float pair or a double).  Gather: the node
     blocks it sums (each of the 6 upper blocks once when the node-block pairs
     are summed once, else the 9 blocks, mirrored ones included), the double
-    CSR values out, the pair lists and slots (3 x 8 per element), per node its
-    dofs, offsets, row length and row pointers, and the column map (2 bytes a
-    row position)."""
+    CSR values out, 32 bytes for each node-block pair, the positions of the
+    contributions beyond two (4 bytes each: 3 blocks an element), per node its six row
+    starts, and the column positions (12 bytes a node block)."""
     from flexshell import _abi
     es = 4 if precision == _abi.FS_MIXED else 8
     el_in = 3 * 4 + 3 * 24 + 3 * 24 + 3 + 8 + (3 * 12 if precision != _abi.FS_FP64 else 0)
     elem = nelem * (el_in + 216 * es)
     blocks = 216 if pairs_once else 324
-    gather = (nelem * blocks * es + nnz * 8 + nelem * 3 * 8 + nodes * (6 * 4 + 8 + 4 + 8 + 6 * 8)
-              + 2 * nnz // 6)
+    nblocks = nnz // 36
+    gather = (nelem * (blocks * es + 3 * 4) + nnz * 8 + (nblocks + nodes) // 2 * 32 + nblocks * 12 + nodes * 6 * 8)
     return elem, gather
 
 

@@ -37,7 +37,8 @@ size_t q4_smem(int precision, bool layered, int epb)
 // The elements per block (the tuned tile) is a launch parameter (block size
 // / 4): every tile runs the same compiled kernel and the same arithmetic.
 // only: null, or the elements to do (a byte each, by rank)
-template <class R, bool COMP, class S>
+// FIXED (layered, double): the Gram products in fixed point
+template <class R, bool COMP, class S, bool FIXED>
 __global__ void __launch_bounds__(128, 2)
     k_q4_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
@@ -177,6 +178,47 @@ __global__ void __launch_bounds__(128, 2)
     }
     }
     __syncwarp();
+    if constexpr (FIXED) {
+        // the element's exponents, then its rows to fixed point, a fourth a lane
+        DofMax mx;
+        if (active) {
+            for (int k = 8 * qp; k < 8 * qp + 8; k++) mx.template row<4>(rows + k * ND);
+            mx.rotations(rows + DR + 3 * qp);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            mx.m[k] = max(mx.m[k], __shfl_xor_sync(0xffffffffu, mx.m[k], 1));
+            mx.m[k] = max(mx.m[k], __shfl_xor_sync(0xffffffffu, mx.m[k], 2));
+        }
+        const bool fixed = active && mx.usable();
+        int E[6];
+        mx.exponents(E, 1);
+        if (fixed) {
+#pragma unroll 1
+            for (int k = 32 * qp; k < 32 * qp + 32; k++)
+#pragma unroll
+                for (int q = 0; q < 6; q++) to_fixed(rows + 6 * k + q, E[q]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) to_fixed(rows + DR + 3 * qp + k, E[3 + k]);
+        }
+        __syncwarp();
+        if (fixed) {
+            double *o = ke + r * (10 * 36);
+            const unsigned swapped = swapped_blocks<4>(m.conn + r * 4);
+            fixed_diagonal<32, ND>(rows, rows + DR + 3 * qp, qp, E, o + ub(qp, qp, 4) * 36);
+#pragma unroll 1
+            for (int t = 0; t < 3; t++) {
+                const int u = qp + 4 * t, ob = u < 6 ? u : u - 6, i0 = u < 6 ? 0 : 3;
+                const int a0 = ob < 3 ? 0 : (ob < 5 ? 1 : 2);
+                const int b0 = ob < 3 ? ob + 1 : (ob < 5 ? ob - 1 : 3);
+                const bool sw = (swapped >> (4 * a0 + b0)) & 1u;
+                double v[3][6];
+                fixed_rows<32, ND, false, 0>(rows, rows, sw ? b0 : a0, sw ? a0 : b0, E, v, i0);
+                store_rows<double, 3>(o + ub(a0, b0, 4) * 36 + 6 * i0, v);
+            }
+            return;
+        }
+    }
     if (!active) return;
     S *out = ke + r * (10 * 36);
     const unsigned swapped = swapped_blocks<4>(m.conn + r * 4);
@@ -230,7 +272,7 @@ __global__ void __launch_bounds__(128, 2)
     }
 }
 
-template <class R, bool COMP, class S = R>
+template <class R, bool COMP, class S = R, bool FIXED = false>
 static int run_q4(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
 {
     int epb = c->tune.elem_epb;
@@ -238,7 +280,7 @@ static int run_q4(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
     const int prec = sizeof(R) == 8 ? FS_FP64 : FS_MIXED;
     while (epb > 16 && q4_smem(prec, COMP, epb) > 227 * 1024) epb /= 2;
     const size_t smem = q4_smem(prec, COMP, epb);
-    auto kern = k_q4_elements<R, COMP, S>;
+    auto kern = k_q4_elements<R, COMP, S, FIXED>;
     FS_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<nblk2(c->mesh.nelem, epb), epb * 4, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status, only);
     FS_CUDA(c, cudaGetLastError());
@@ -254,7 +296,7 @@ int run_q4_any(fs_ctx *c, int precision, void *ke)
     const bool comp = c->mesh.etype == FS_Q4RSCOMP;
     if (precision == FS_FP64) {
         double *k = (double *)ke;
-        if (comp) return run_q4<double, true>(c, k);
+        if (comp) return c->drops_zeros ? run_q4<double, true>(c, k) : run_q4<double, true, double, true>(c, k);
         return c->drops_zeros ? run_q4<double, false>(c, k) : run_fp64(c, k);
     }
     if (precision == FS_MIXED_COMP) {

@@ -20,7 +20,8 @@ template <class R, bool COMP, bool AVGK, class S> struct T3MinBlocks {
 };
 
 // only: null, or the elements to do (a byte each, by rank)
-template <class R, bool COMP, bool AVGK, class S>
+// FIXED (layered, double): the Gram products in fixed point
+template <class R, bool COMP, bool AVGK, class S, bool FIXED>
 __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     k_t3_elements(const MeshDev m, const MatConst mc, S *ke, int *status, const uint8_t *only)
 {
@@ -40,13 +41,31 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     int st = t3_rows<R, COMP, AVGK, true>(in, mc, gc, rows, ND);
     if (st) atomicOr(status, DEV_NEG_DRILL);
     const unsigned swapped = swapped_blocks<3>(m.conn + r * 3);
+    if constexpr (FIXED) {
+        typedef LayeredRows<3, 6 + NS> L;
+        DofMax mx;
+        for (int k = 0; k < 6 + NS; k++) mx.template row<3>(rows + k * ND);
+        for (int k = 0; k < 3; k++) mx.rotations(rows + L::DR + 3 * k);
+        if (mx.usable()) {
+            int E[6];
+            mx.exponents(E, 0);
+#pragma unroll 1
+            for (int k = 0; k < 3 * (6 + NS); k++)
+#pragma unroll
+                for (int q = 0; q < 6; q++) to_fixed(rows + 6 * k + q, E[q]);
+#pragma unroll
+            for (int k = 0; k < 9; k++) to_fixed(rows + L::DR + k, E[3 + k % 3]);
+            write_blocks_fixed<3, 6 + NS>(rows, E, swapped, ke + r * (6 * 36));
+            return;
+        }
+    }
     if constexpr (COMP)
         write_blocks_layered<R, S, 3, 6 + NS>(rows, swapped, ke + r * (6 * 36));
     else
         write_blocks_compact<R, S, 3, NS>(rows, swapped, ke + r * (6 * 36));
 }
 
-template <class R, bool COMP, bool AVGK, class S = R>
+template <class R, bool COMP, bool AVGK, class S = R, bool FIXED = false>
 static int run_t3(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
 {
     int epb = c->tune.elem_epb;
@@ -54,7 +73,7 @@ static int run_t3(fs_ctx *c, S *ke, const uint8_t *only = nullptr)
     if (epb != 32 && epb != 64) epb = 128;
     if (sizeof(R) == 8 && AVGK && epb > 64) epb = 64;  // shared memory of the double average-K rows
     const size_t smem = t3_smem(sizeof(R) == 8 ? FS_FP64 : FS_MIXED, AVGK, COMP, epb);
-    auto kern = k_t3_elements<R, COMP, AVGK, S>;
+    auto kern = k_t3_elements<R, COMP, AVGK, S, FIXED>;
     FS_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<nblk2(c->mesh.nelem, epb), epb, smem, c->stream>>>(c->mesh, c->mc, ke, c->d_status, only);
     FS_CUDA(c, cudaGetLastError());
@@ -71,7 +90,9 @@ int run_t3_any(fs_ctx *c, int precision, void *ke)
     const bool avgk = c->params.transv_shear_formulation == 1;
     if (precision == FS_FP64) {
         double *k = (double *)ke;
-        if (comp) return avgk ? run_t3<double, true, true>(c, k) : run_t3<double, true, false>(c, k);
+        if (comp && c->drops_zeros) return avgk ? run_t3<double, true, true>(c, k) : run_t3<double, true, false>(c, k);
+        if (comp)
+            return avgk ? run_t3<double, true, true, double, true>(c, k) : run_t3<double, true, false, double, true>(c, k);
         if (avgk) return run_t3<double, false, true>(c, k);
         return c->drops_zeros ? run_t3<double, false, false>(c, k) : run_fp64(c, k);
     }
