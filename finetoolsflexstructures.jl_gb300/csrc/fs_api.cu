@@ -1,4 +1,7 @@
 // C ABI of the flexshell library (include/flexshell.h).
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <string.h>
 
 #include <algorithm>
@@ -49,6 +52,27 @@ int read_status(fs_ctx *c, int *bits)
     if (h) FS_CUDA(c, cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
     *bits = h;
     return FS_OK;
+}
+
+// Device memory to the caller's.  A large result usually goes to memory that the
+// caller has just allocated, and a device copy into pages that do not exist yet
+// faults them in one by one (38 MB: 24 ms); the system makes them all at once (1.2
+// ms with the copy).  The contents of existing pages stay.
+int copy_out(fs_ctx *c, void *dst, const void *src, size_t bytes)
+{
+    const size_t POPULATE_LEAST = 1 << 20;
+    if (bytes >= POPULATE_LEAST) {
+        cudaPointerAttributes at{};
+        const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        if (pageable) {
+            const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), b = ((uintptr_t)dst + page - 1) / page * page,
+                            e = ((uintptr_t)dst + bytes) / page * page;
+            const int populate_write = 23;  // MADV_POPULATE_WRITE; a kernel without it refuses, and the copy does the work
+            if (e > b) (void)madvise((void *)b, e - b, populate_write);
+        }
+    }
+    return cuda_check(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream), "copy to the host");
 }
 
 static void free_pattern(PatternDev &P)
@@ -615,15 +639,15 @@ int fs_matrix_copy(fs_ctx *c, int64_t *colptr, int64_t *rowval, double *nzval)
     if (colptr) {
         k_plus_one_i64<<<(unsigned)((n + 1 + 255) / 256), 256, 0, c->stream>>>(n + 1, c->mat_rowptr, c->stage64);
         FS_CUDA(c, cudaGetLastError());
-        FS_CUDA(c, cudaMemcpyAsync(colptr, c->stage64, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, c->stream));
+        FS_TRY(copy_out(c, colptr, c->stage64, sizeof(int64_t) * (n + 1)));
         FS_CUDA(c, cudaStreamSynchronize(c->stream));
     }
     if (rowval && nnz) {
         k_plus_one_i32<<<(unsigned)((nnz + 255) / 256), 256, 0, c->stream>>>(nnz, c->mat_colidx, c->stage64);
         FS_CUDA(c, cudaGetLastError());
-        FS_CUDA(c, cudaMemcpyAsync(rowval, c->stage64, sizeof(int64_t) * nnz, cudaMemcpyDeviceToHost, c->stream));
+        FS_TRY(copy_out(c, rowval, c->stage64, sizeof(int64_t) * nnz));
     }
-    if (nzval && nnz) FS_CUDA(c, cudaMemcpyAsync(nzval, c->vals, sizeof(double) * nnz, cudaMemcpyDeviceToHost, c->stream));
+    if (nzval && nnz) FS_TRY(copy_out(c, nzval, c->vals, sizeof(double) * nnz));
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     return FS_OK;
 }
@@ -639,10 +663,10 @@ int fs_matrix_copy_i32(fs_ctx *c, int32_t *colptr, int32_t *rowval, double *nzva
         FS_TRY(ensure_scratch(c, sizeof(int32_t) * (size_t)(n + 1)));
         k_to_i32<<<(unsigned)((n + 1 + 255) / 256), 256, 0, c->stream>>>(n + 1, c->mat_rowptr, (int32_t *)c->scratch);
         FS_CUDA(c, cudaGetLastError());
-        FS_CUDA(c, cudaMemcpyAsync(colptr, c->scratch, sizeof(int32_t) * (size_t)(n + 1), cudaMemcpyDeviceToHost, c->stream));
+        FS_TRY(copy_out(c, colptr, c->scratch, sizeof(int32_t) * (size_t)(n + 1)));
     }
-    if (rowval && nnz) FS_CUDA(c, cudaMemcpyAsync(rowval, c->mat_colidx, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream));
-    if (nzval && nnz) FS_CUDA(c, cudaMemcpyAsync(nzval, c->vals, sizeof(double) * (size_t)nnz, cudaMemcpyDeviceToHost, c->stream));
+    if (rowval && nnz) FS_TRY(copy_out(c, rowval, c->mat_colidx, sizeof(int32_t) * (size_t)nnz));
+    if (nzval && nnz) FS_TRY(copy_out(c, nzval, c->vals, sizeof(double) * (size_t)nnz));
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     return FS_OK;
 }

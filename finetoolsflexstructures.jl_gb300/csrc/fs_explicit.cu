@@ -990,9 +990,9 @@ int fs_explicit_get_state(fs_ctx *c, double *U, double *V, double *A)
     auto &x = c->ex;
     if (!x.ready) return set_err(c, FS_ERR_STATE, "call fs_explicit_setup first");
     size_t bn = sizeof(double) * (size_t)x.n;
-    if (U) FS_CUDA(c, cudaMemcpyAsync(U, x.U, bn, cudaMemcpyDeviceToHost, c->stream));
-    if (V) FS_CUDA(c, cudaMemcpyAsync(V, x.V, bn, cudaMemcpyDeviceToHost, c->stream));
-    if (A) FS_CUDA(c, cudaMemcpyAsync(A, x.A, bn, cudaMemcpyDeviceToHost, c->stream));
+    if (U) FS_TRY(copy_out(c, U, x.U, bn));
+    if (V) FS_TRY(copy_out(c, V, x.V, bn));
+    if (A) FS_TRY(copy_out(c, A, x.A, bn));
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     return FS_OK;
 }

@@ -264,6 +264,7 @@ int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *co
 int exclusive_scan_i64(fs_ctx *c, const int64_t *in, int64_t *out, int64_t n, int64_t *total);
 int ensure_scratch(fs_ctx *c, size_t bytes);
 int read_status(fs_ctx *c, int *bits);
+int copy_out(fs_ctx *c, void *dst, const void *src, size_t bytes);
 // FS_OK when the context holds a shell mesh with parameters (and, with
 // need_dofs, a dof numbering) and its layups if layered; else the error code
 int check_ready(fs_ctx *c, bool need_dofs = true);

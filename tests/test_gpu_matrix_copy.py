@@ -39,3 +39,25 @@ def test_the_same_matrix(assembler, n, free):
     femm.ctx.call("fs_matrix_copy_i32", None, None, ptr(v))
     assert np.array_equal(v, v64)
     femm.close()
+
+
+def test_large_copies_into_any_memory():
+    # results of a megabyte and more: into new pages, used ones, and an address
+    # inside a page, with what lies around them untouched
+    xyz, conn, dof, nfree = PB.jittered_plate(60, False, wavy=0.02, seed=2)
+    femm = F.FEMMShellT3FF(conn, 0.01, F.materials.MatDeforElastIso(200e9, 0.3, 7850.0))
+    geom0 = F.NodalField(xyz)
+    dchi = F.NodalField(np.zeros((len(xyz), 6)))
+    dchi.dofnums = np.asfortranarray(dof)
+    femm.associategeometry(geom0)
+    K = femm.stiffness(F.SysmatAssemblerSparse(), geom0, None, None, dchi)
+    z = K.nnz
+    assert 8 * z > 1 << 20
+    for shift in (0, 1, 511):
+        for fill in (None, -7.0):
+            buf = np.empty(z + 1024) if fill is None else np.full(z + 1024, fill)
+            buf[:shift], buf[shift + z:] = 3.0, 4.0
+            femm.ctx.call("fs_matrix_copy_i32", None, None, ptr(buf[shift:]))
+            assert np.array_equal(buf[shift:shift + z], K.data)
+            assert (buf[:shift] == 3.0).all() and (buf[shift + z:] == 4.0).all()
+    femm.close()
