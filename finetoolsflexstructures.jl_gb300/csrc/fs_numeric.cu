@@ -307,7 +307,7 @@ int assemble_mass(fs_ctx *c, int assembler, int64_t n)
         c->mat_colidx = P.diag_colidx;
         c->mat_nnz = n;
         if (assembler == FS_ASM_SPARSE_SYMM)
-            return compact_zeros(c, n, P.diag_rowptr, P.diag_colidx, n);
+            FS_TRY(compact_zeros(c, n, P.diag_rowptr, P.diag_colidx, n));
     }
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     return FS_OK;

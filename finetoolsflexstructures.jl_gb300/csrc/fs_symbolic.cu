@@ -81,8 +81,18 @@ __global__ void k_scan_sums(int64_t *sums, int64_t nchunks)
     if (threadIdx.x == 0) sums[nchunks] = carry;
 }
 
+// SUMMED: sums is scanned already (with the total behind); otherwise each block adds
+// up the chunks before its own
+template <bool SUMMED>
 __global__ void k_chunk_scan(const int64_t *in, int64_t n, const int64_t *sums, int64_t *out)
 {
+    int64_t before = 0, unused;
+    if (SUMMED) {
+        before = sums[blockIdx.x];
+    } else {
+        for (int64_t k = threadIdx.x; k < (int64_t)blockIdx.x; k += SCAN_TPB) before += sums[k];
+        before = block_excl_scan(before, unused);
+    }
     int64_t base = (int64_t)blockIdx.x * SCAN_CHUNK + (int64_t)threadIdx.x * SCAN_ITEMS;
     int64_t v[SCAN_ITEMS];
     int64_t s = 0;
@@ -92,19 +102,19 @@ __global__ void k_chunk_scan(const int64_t *in, int64_t n, const int64_t *sums, 
         s += v[i];
     }
     int64_t ex;
-    block_excl_scan(s, ex);
-    int64_t run = sums[blockIdx.x] + ex;
+    const int64_t own = block_excl_scan(s, ex);
+    int64_t run = before + ex;
     for (int i = 0; i < SCAN_ITEMS; i++) {
         int64_t k = base + i;
         if (k < n) out[k] = run;
         run += v[i];
     }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = before + own;
 }
 
-__global__ void k_set_total(int64_t *out, int64_t n, const int64_t *sums, int64_t nchunks)
-{
-    out[n] = sums[nchunks];
-}
+// Up to this many chunks their sums are added up by every block, which saves a
+// launch (2 us of a small assembly's 200) for at most a megabyte of reads from L2.
+static const int64_t SCAN_DIRECT_CHUNKS = 512;
 
 int exclusive_scan_i64(fs_ctx *c, const int64_t *in, int64_t *out, int64_t n, int64_t *total)
 {
@@ -113,9 +123,12 @@ int exclusive_scan_i64(fs_ctx *c, const int64_t *in, int64_t *out, int64_t n, in
     FS_TRY(ensure_scratch(c, sizeof(int64_t) * (nchunks + 1)));
     int64_t *sums = (int64_t *)c->scratch;
     k_chunk_sums<<<(unsigned)nchunks, SCAN_TPB, 0, c->stream>>>(in, n, sums);
-    k_scan_sums<<<1, SCAN_TPB, 0, c->stream>>>(sums, nchunks);
-    k_chunk_scan<<<(unsigned)nchunks, SCAN_TPB, 0, c->stream>>>(in, n, sums, out);
-    k_set_total<<<1, 1, 0, c->stream>>>(out, n, sums, nchunks);
+    if (nchunks <= SCAN_DIRECT_CHUNKS) {
+        k_chunk_scan<false><<<(unsigned)nchunks, SCAN_TPB, 0, c->stream>>>(in, n, sums, out);
+    } else {
+        k_scan_sums<<<1, SCAN_TPB, 0, c->stream>>>(sums, nchunks);
+        k_chunk_scan<true><<<(unsigned)nchunks, SCAN_TPB, 0, c->stream>>>(in, n, sums, out);
+    }
     FS_CUDA(c, cudaGetLastError());
     if (total) {
         FS_CUDA(c, cudaMemcpyAsync(total, out + n, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
@@ -648,7 +661,7 @@ __global__ void k_compact(int64_t n, const int64_t *__restrict__ rowptr, const i
 }
 
 // The matrix without its exact zeros: the kept entries go to a second pair of
-// buffers, and the two value buffers change places
+// buffers, and the two value buffers change places.  The caller waits for it.
 int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *colidx, int64_t nnz)
 {
     FS_TRY(grow(c, &c->pat.tmp_cnt, &c->pat.cap_tmp_cnt, (size_t)n));
@@ -676,7 +689,6 @@ int compact_zeros(fs_ctx *c, int64_t n, const int64_t *rowptr, const int32_t *co
         std::swap(c->vals_cap, c->cmp_vals_cap);
     } else
         FS_CUDA(c, cudaMemcpyAsync(c->vals, c->cmp_vals, sizeof(double) * nnz2, cudaMemcpyDeviceToDevice, c->stream));
-    FS_CUDA(c, cudaStreamSynchronize(c->stream));
     c->mat_rowptr = c->cmp_rowptr;
     c->mat_colidx = c->cmp_colidx;
     c->mat_nnz = nnz2;

@@ -22,6 +22,22 @@ def _kept(K):
     return K
 
 
+@pytest.mark.parametrize("n", [12, 13, 294, 296])
+def test_row_counts_around_the_scans_forms(n):
+    # the row lengths are summed in chunks of 1,024 rows: one chunk and two, and on
+    # either side of 512 chunks (6 dofs a node, (n + 1)^2 nodes)
+    xyz, conn, dof, nfree = PB.jittered_plate(n, True, wavy=0.0, seed=1)
+    femm = F.FEMMShellQ4RS(conn, 0.01, F.materials.MatDeforElastIso(200e9, 0.3, 7850.0))
+    geom0 = F.NodalField(xyz)
+    dchi = F.NodalField(np.zeros((len(xyz), 6)))
+    dchi.numberdofs()
+    femm.associategeometry(geom0)
+    A = femm.stiffness(F.SysmatAssemblerSparse(), geom0, None, None, dchi, precision=F.FS_MIXED)
+    B = femm.stiffness(F.SysmatAssemblerSparseSymm(), geom0, None, None, dchi, precision=F.FS_MIXED)
+    _same(_kept(A), B)
+    femm.close()
+
+
 @pytest.mark.parametrize("quads", [False, True])
 @pytest.mark.parametrize("n", [1, 2, 5, 17, 40])
 @pytest.mark.parametrize("wavy", [0.0, 0.03])
