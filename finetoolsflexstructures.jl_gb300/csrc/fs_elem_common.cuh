@@ -366,7 +366,7 @@ struct DofMax {
     __device__ __forceinline__ void exponents(int (&E)[6], int spare) const
     {
 #pragma unroll
-        for (int k = 0; k < 6; k++) E[k] = (m[k] ? fx_exp(m[k]) : 0) + spare;
+        for (int k = 0; k < 6; k++) E[k] = fx_group(m[k]) + spare;
     }
 };
 // a double in shared memory replaced by its fixed-point number

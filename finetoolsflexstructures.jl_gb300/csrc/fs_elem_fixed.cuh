@@ -57,16 +57,16 @@ struct FxExp {
 FS_HD FxExp fx_exponents(const FxMax &mx, int spare)
 {
     FxExp x;
-    x.cm = fx_exp(mx.m) + spare;
-    x.r = fx_exp(mx.r) + spare;
-    x.u = fx_exp(mx.u) + spare;
-    x.g = fx_exp(mx.g);
+    x.cm = fx_group(mx.m) + spare;
+    x.r = fx_group(mx.r) + spare;
+    x.u = fx_group(mx.u) + spare;
+    x.g = fx_group(mx.g);
     x.h = x.u + x.g;
     x.coupled = mx.u != 0;
     // |w e2 + sum h t| stays below 1.2 of the group: |w| below a half, |h| below
     // three eighths in each component
-    const int w = fx_exp(mx.w);
-    x.t = (x.coupled && x.h + 2 > w ? x.h + 2 : w) + 1;
+    const int w = fx_group(mx.w);
+    x.t = (x.coupled && (x.h + 2 > w || mx.w == 0) ? x.h + 2 : w) + 1;
     FS_UNROLL
     for (int c = 0; c < 3; c++) {
         x.em[c] = fx_exp(mx.e[c]) > -60 ? fx_exp(mx.e[c]) : -60;  // below 2^-60 of the unit: counts as that

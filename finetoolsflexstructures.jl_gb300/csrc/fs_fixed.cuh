@@ -86,14 +86,18 @@ FS_HD void fx_max(uint32_t &mx, double x)
     const uint32_t u = fx_hi(x) & 0x7fffffffu;
     mx = u > mx ? u : mx;
 }
-// the group's exponent: every |x| of it is below 2^E
+// the exponent of numbers that are not all zero: every |x| of them is below 2^E
 FS_HD int fx_exp(uint32_t mx) { return (int)(mx >> 20) - 1022; }
+// the group's exponent; of a group of zeros (a thickness or a material stiffness
+// that vanishes) one at which they stay zeros
+FS_HD int fx_group(uint32_t mx) { return mx ? fx_exp(mx) : 0; }
 // finite, and products of four such groups are normal doubles to their last
 // bit (a group of zeros counts as usable)
 FS_HD bool fx_usable(uint32_t mx) { return mx < (uint32_t)(1023 + 200) << 20 && (mx == 0 || mx > (uint32_t)(1023 - 200) << 20); }
 
 // X of x in a group of exponent E (towards zero); |x| = 2^E exactly (a unit
-// vector's 1.0 in exponent 0) is taken too
+// vector's 1.0 in exponent 0) is taken too.  A zero is shifted out where E is
+// above -960, as every group's exponent is
 FS_HD int64_t fx_int(double x, int E)
 {
     const uint32_t hi = fx_hi(x);
