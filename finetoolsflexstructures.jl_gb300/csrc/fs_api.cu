@@ -301,6 +301,7 @@ int fs_mesh_set(fs_ctx *c, int elem_type, int64_t nnodes, const double *xyz, int
     FS_CUDA(c, cudaStreamSynchronize(c->stream));
     free_mesh(c->mesh);
     reset_pattern(c->pat);
+    c->fx_asked = 0;  // a row buffer that came out small for the previous mesh is asked for again
     c->mat_rowptr = nullptr;
     free_shift(c);  // a factor of the previous mesh's stiffness
     free_beam(c);

@@ -26,11 +26,11 @@
 
 #include "fs_elem_common.cuh"
 #include "fs_elem_fixed.cuh"
+#include "fs_fp64_rows.h"
 
 namespace fs {
 
 static const size_t FX_CHUNK_BYTES = (size_t)1 << 30;  // rows of a chunk
-static const int64_t FX_LEAST_GROUPS = 608;            // of 32 elements: four blocks of the Gram kernel an SM
 
 // slots of an element: its rows, then its exponents (m0, m1) (m2, t) (r, done elsewhere)
 constexpr int T3_SLOTS = CompactRows<3, 2>::SIZE + 3;
@@ -281,36 +281,34 @@ static int64_t chunk_elements(const MeshDev &m)
 // slots that the marks of the elements to do in double take, ahead of the rows
 static size_t mark_slots(const MeshDev &m) { return ((size_t)m.nelem + 255) / 256 * (256 / sizeof(FxSlot)); }
 
-// The buffer of the marks and of a chunk's rows, kept by the context.  Where the
-// memory for a whole chunk is not there, half of it is tried, and so on; with no
-// memory for the smallest, fx_rows stays null.
+// The buffer of the marks and of a chunk's rows, kept by the context.  With no
+// memory for the smallest chunk, fx_rows stays null.
 int ensure_fp64_rows(fs_ctx *c)
 {
     const MeshDev &m = c->mesh;
     if (m.etype != FS_T3FF && m.etype != FS_Q4RS) return FS_OK;
-    const size_t group = (size_t)FX_GROUP * (m.nen == 3 ? T3_SLOTS : Q4_SLOTS), marks = mark_slots(m);
-    size_t want = (size_t)chunk_elements(m) / FX_GROUP;
-    if (c->fx_rows && c->fx_asked >= marks + want * group) return FS_OK;
-    c->fx_asked = marks + want * group;
-    for (FxSlot *rows = (FxSlot *)c->fx_rows;; want /= 2) {
-        const int st = grow(c, &rows, &c->cap_fx_rows, marks + want * group);
-        c->fx_rows = rows;
-        if (st != FS_ERR_OOM) return st;
-        if (want <= (size_t)FX_LEAST_GROUPS) return FS_OK;
-    }
+    const size_t group = (size_t)FX_GROUP * (m.nen == 3 ? T3_SLOTS : Q4_SLOTS);
+    return fx_reserve(c->fx_rows ? c->cap_fx_rows : 0, c->fx_asked, mark_slots(m), (size_t)chunk_elements(m) / FX_GROUP, group,
+                      FS_OK, FS_ERR_OOM, [&](size_t slots) {
+                          FxSlot *rows = (FxSlot *)c->fx_rows;
+                          const int st = grow(c, &rows, &c->cap_fx_rows, slots);
+                          c->fx_rows = rows;
+                          return st;
+                      });
 }
 
 int run_fp64(fs_ctx *c, double *ke)
 {
     const MeshDev &m = c->mesh;
     const bool t3 = m.nen == 3;
-    FS_TRY(ensure_fp64_rows(c));
-    if (!c->fx_rows) return t3 ? redo_t3(c, ke, nullptr) : redo_q4(c, ke, nullptr);
-    const size_t marks = mark_slots(m);
+    // (the allocation-free path has the buffer, or none, from its pattern on)
+    if (ke != c->noalloc_scratch) FS_TRY(ensure_fp64_rows(c));
+    const size_t marks = mark_slots(m), group = (size_t)FX_GROUP * (t3 ? T3_SLOTS : Q4_SLOTS);
+    const int64_t held = c->fx_rows ? (int64_t)fx_groups_held(c->cap_fx_rows, marks, group) * FX_GROUP : 0;
+    if (!held) return t3 ? redo_t3(c, ke, nullptr) : redo_q4(c, ke, nullptr);
     uint8_t *redo = (uint8_t *)c->fx_rows;
     FxSlot *rows = (FxSlot *)c->fx_rows + marks;
-    const int64_t fit = (int64_t)((c->cap_fx_rows - marks) / ((size_t)FX_GROUP * (t3 ? T3_SLOTS : Q4_SLOTS))) * FX_GROUP;
-    const int64_t chunk = std::min(chunk_elements(m), fit);
+    const int64_t chunk = std::min(chunk_elements(m), held);
     int epb = c->tune.elem_epb;
     if (t3 && epb != 32 && epb != 64) epb = 128;
     if (!t3 && epb != 8 && epb != 16) epb = 32;

@@ -21,7 +21,7 @@ SOURCES = ["fs_api.cu", "fs_symbolic.cu", "fs_numeric.cu", "fs_elem_t3.cu", "fs_
            "fs_loads.cu", "fs_eigen.cu"]
 HEADERS = ["fs_internal.cuh", "fs_elem_math.cuh", "fs_elem_common.cuh", "fs_elem_fixed.cuh",
            "fs_fixed.cuh", "fs_comp_sum.cuh", "fs_beam_math.cuh",
-           "fs_host_prep.h"]
+           "fs_host_prep.h", "fs_fp64_rows.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
