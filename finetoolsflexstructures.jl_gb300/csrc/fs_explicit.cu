@@ -400,10 +400,12 @@ struct CdStep {
 };
 
 // NEXT: also the displacement of the next step, copied to `xn`; UN blocks at a
-// time, their loads and those of the next ones' items in flight together
+// time, their loads and those of the next ones' items in flight together.  The
+// kernel may start while the step before still writes `xp`: no restrict, which
+// would let the compiler take it for read-only, and only plain loads of it
 template <int PREC, bool NEXT, int UN>
-__global__ void __launch_bounds__(UN == 1 ? CD_ONE_BLOCK_TPB : cd_small_tpb(PREC)) k_cd_step(CdStep s, const typename CdTypes<PREC>::X *__restrict__ xp,
-                                                          typename CdTypes<PREC>::X *__restrict__ xn, CdLoad ld)
+__global__ void __launch_bounds__(UN == 1 ? CD_ONE_BLOCK_TPB : cd_small_tpb(PREC)) k_cd_step(CdStep s, const typename CdTypes<PREC>::X *xp,
+                                                          typename CdTypes<PREC>::X *xn, CdLoad ld)
 {
     using V = typename CdTypes<PREC>::V;
     const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, r = th / 3;
