@@ -8,12 +8,27 @@
 // node; and the largest magnitude of each kind.  Then, in fixed point, every row
 // is expanded in place: the coefficients with the element basis and the
 // nodal triads, whose entries are at most one, so that no row entry exceeds its
-// group by more than the expansion's own factor.  Row entries come in five
-// groups with an exponent each, for all rows and nodes of the element: the
-// translations of the membrane rows along each global axis (M), those of the
-// others (T), and the rotations (R).  An exponent for each axis keeps the small
+// group by more than the expansion's own factor.  Row entries come in groups with
+// an exponent each, for all rows of the element: each node's translations in the
+// membrane rows along each global axis (M), those in the others (T) and its
+// rotations (R), and the drilling rows.  An exponent for each axis keeps the small
 // components of an element near a coordinate plane: its membrane rows along the
-// normal must not disturb the much smaller bending stiffness there.
+// normal must not disturb the much smaller bending stiffness there.  One for each
+// node keeps the entries of a node with small gradients, as an elongated element
+// has: an entry of K is off by a few 2^-58 of its two diagonal entries' mean.
+//
+// That is as near as double only while the rows of one node differ by no more than
+// the five bits that 58 has beyond 53, so a triangle longer than T3_LONGEST is left
+// to the double kernel.  Errors of the energies of constant strains, fixed point over
+// double, in the mean of 600 random triangles, the worst of nine energies, by
+// elongation (longest edge squared over twice the area): at most 1.1 up to 32, 1.4
+// from 32 to 64, 2.2 from 64 to 128 (a rotation's shear energy on an axis-aligned
+// plate); with one exponent for all nodes 1.7 from 4 to 8, 2.7 from 16 to 32.
+// Quadrilaterals: 1.9 at most at any elongation, and the matrix is nearer than
+// double's (16 to 1: 0.4 of its error, 256 to 1: 0.002), whose own rows lose more;
+// none is left.  Exponents by node cost 3 % (elements, triangles, 700 x 700: 1.53 and
+// 1.58 ms, quads, 360 x 360: 1.54 and 1.59); a plate of nothing but long triangles takes
+// 5.0 ms instead of 2.05 (4.8 when all was double).
 #pragma once
 
 #include "fs_elem_math.cuh"
@@ -37,41 +52,53 @@ struct TriadFx {
     fx a00, a01, a11, a02, a12, a22;
 };
 
+constexpr double T3_LONGEST = 32;  // longest edge squared over twice the area
+
 // Coefficient maxima (high words) of one element, and the exponents from them.
 struct FxMax {
-    uint32_t m = 0, w = 0, r = 0, u = 0, g = 0;  // u,v | w | r0,r1,drilling | mu | gradients
-    uint32_t e[3] = {0, 0, 0};                   // e0, e1 along each axis
+    uint32_t m[4] = {0, 0, 0, 0}, w[4] = {0, 0, 0, 0};  // of each node: u, v | w
+    uint32_t q[4] = {0, 0, 0, 0}, g[4] = {0, 0, 0, 0};  // r0, r1 | gradients
+    uint32_t r = 0, u = 0;                              // drilling rows | mu
+    uint32_t e[3] = {0, 0, 0};                          // e0, e1 along each axis
     FS_HD bool usable() const
     {
-        return fx_usable(m) && fx_usable(w) && fx_usable(r) && fx_usable(u) && fx_usable(g);
+        bool ok = fx_usable(r) && fx_usable(u);
+        FS_UNROLL
+        for (int j = 0; j < 4; j++) ok = ok && fx_usable(m[j]) && fx_usable(w[j]) && fx_usable(q[j]) && fx_usable(g[j]);
+        return ok;
     }
 };
+// a node's groups M (without the axis'), T and R
+struct FxNode {
+    int m, t, q;
+};
 struct FxExp {
-    int m[3], t, r;     // groups M (by axis), T and R
-    int em[3];          // units: e0, e1 along each axis
-    int cm;             // membrane coefficients
-    int u, g, h;        // mu, gradients, and the drilling coupling's h (u + g)
-    bool coupled;       // some mu is not zero
+    int m[4], t[4], q[4], g[4];  // each node's groups, and gradients
+    int em[3];                   // units: e0, e1 along each axis
+    int r, u;                    // drilling rows, mu
+    bool coupled;                // some mu is not zero
+    FS_HD FxNode node(int j) const { return FxNode{m[j], t[j], q[j]}; }
 };
 // spare: bits kept free for the longer sums of an element with several points
 FS_HD FxExp fx_exponents(const FxMax &mx, int spare)
 {
     FxExp x;
-    x.cm = fx_group(mx.m) + spare;
     x.r = fx_group(mx.r) + spare;
     x.u = fx_group(mx.u) + spare;
-    x.g = fx_group(mx.g);
-    x.h = x.u + x.g;
     x.coupled = mx.u != 0;
-    // |w e2 + sum h t| stays below 1.2 of the group: |w| below a half, |h| below
-    // three eighths in each component
-    const int w = fx_group(mx.w);
-    x.t = (x.coupled && (x.h + 2 > w || mx.w == 0) ? x.h + 2 : w) + 1;
     FS_UNROLL
-    for (int c = 0; c < 3; c++) {
-        x.em[c] = fx_exp(mx.e[c]) > -60 ? fx_exp(mx.e[c]) : -60;  // below 2^-60 of the unit: counts as that
-        x.m[c] = x.cm + x.em[c];
+    for (int j = 0; j < 4; j++) {
+        x.m[j] = fx_group(mx.m[j]) + spare;
+        x.q[j] = fx_group(mx.q[j]) + spare;
+        x.g[j] = fx_group(mx.g[j]);
+        // |w e2 + sum h t| stays below 1.2 of the group: |w| below a half, |h| below
+        // three eighths in each component (h: u + g, the drilling coupling)
+        const int w = fx_group(mx.w[j]), h = x.u + x.g[j] + 2;
+        x.t[j] = (x.coupled && (h > w || mx.w[j] == 0) ? h : w) + 1;
     }
+    FS_UNROLL
+    for (int c = 0; c < 3; c++)
+        x.em[c] = fx_exp(mx.e[c]) > -60 ? fx_exp(mx.e[c]) : -60;  // below 2^-60 of the unit: counts as that
     return x;
 }
 
@@ -143,6 +170,7 @@ FS_HD void triad_axes(const TriadFx &A, const fx e[3][3], fx t[3][3])
 union FxSlot {
     double d;
     fx x;
+    int16_t s[4];
 };
 constexpr int FX_GROUP = 32;
 struct FxSlots {
@@ -152,13 +180,13 @@ struct FxSlots {
 };
 
 // Membrane row in place: [u0 v0 u1 v1 ..] -> NN x 3 translations
-template <int NN> FS_HD void expand_membrane(FxSlots row, const fx em[2][3], int cm)
+template <int NN> FS_HD void expand_membrane(FxSlots row, const fx em[2][3], const FxExp &ex)
 {
     fx u[NN], v[NN];
     FS_UNROLL
     for (int j = 0; j < NN; j++) {
-        u[j] = fx_make(row[2 * j].d, cm);
-        v[j] = fx_make(row[2 * j + 1].d, cm);
+        u[j] = fx_make(row[2 * j].d, ex.m[j]);
+        v[j] = fx_make(row[2 * j + 1].d, ex.m[j]);
     }
     FS_UNROLL
     for (int j = 0; j < NN; j++)
@@ -171,7 +199,7 @@ template <int NN> FS_HD void expand_membrane(FxSlots row, const fx em[2][3], int
 }
 
 // Bending or shear row in place: [w0.. | r0 r1 per node | mu0..] -> NN x 6
-// (translations, rotations).  g: the basis gradients (exponent ex.g).
+// (translations, rotations).  g: the basis gradients (exponents ex.g).
 template <int NN>
 FS_HD void expand_bending(FxSlots row, bool has_w, const fx e2[3], const fx t[NN][3][3], const TriadFx A[NN],
                           const fx g[NN][2], const FxExp &ex)
@@ -180,9 +208,9 @@ FS_HD void expand_bending(FxSlots row, bool has_w, const fx e2[3], const fx t[NN
     FS_UNROLL
     for (int j = 0; j < NN; j++) {
         w[j] = fx{0, 0};
-        if (has_w) w[j] = fx_make(row[j].d, ex.t);
-        r0[j] = fx_make(row[NN + 2 * j].d, ex.r);
-        r1[j] = fx_make(row[NN + 2 * j + 1].d, ex.r);
+        if (has_w) w[j] = fx_make(row[j].d, ex.t[j]);
+        r0[j] = fx_make(row[NN + 2 * j].d, ex.q[j]);
+        r1[j] = fx_make(row[NN + 2 * j + 1].d, ex.q[j]);
     }
     if (ex.coupled) {
         // P_r = sum_i mu_i A_i[r][:], h_j = (g_jx P_1 - g_jy P_0) / 2
@@ -209,15 +237,16 @@ FS_HD void expand_bending(FxSlots row, bool has_w, const fx e2[3], const fx t[NN
             P[0][k] = fx_done(s[0][k]);
             P[1][k] = fx_done(s[1][k]);
         }
-        const int sh = ex.t - ex.h + 1;  // to the group's exponent, and the half
         FS_UNROLL
-        for (int j = 0; j < NN; j++)
+        for (int j = 0; j < NN; j++) {
+            const int sh = ex.t[j] - (ex.u + ex.g[j]) + 1;  // to the group's exponent, and the half
             FS_UNROLL
             for (int k = 0; k < 3; k++) {
                 FxSum q = fx_mul(g[j][0], P[1][k]);
                 fx_mac(q, fx_neg(g[j][1]), P[0][k]);
                 h[j][k] = fx_split(fx_shift(fx_round(q), sh));
             }
+        }
     }
     FS_UNROLL
     for (int j = 0; j < NN; j++)
@@ -241,9 +270,14 @@ template <int NN> struct FxGeom {
     Triad A[NN];
     double g[NN][2];   // basis gradients
 };
-// maxima of the basis components
+// maxima of the basis components and gradients
 template <int NN> FS_HD void fx_max_basis(FxMax &mx, const FxGeom<NN> &geo)
 {
+    FS_UNROLL
+    for (int j = 0; j < NN; j++) {
+        fx_max(mx.g[j], geo.g[j][0]);
+        fx_max(mx.g[j], geo.g[j][1]);
+    }
     FS_UNROLL
     for (int c = 0; c < 3; c++) {
         fx_max(mx.e[c], geo.e[0][c]);
@@ -276,8 +310,10 @@ FS_HD void unit_vector(const double v[3], double e[3], double &len, double &inv)
 // layout).  In the element frame the first edge lies on x: with A, C, D its
 // length and the third node's coordinates, the averaged DSG shear rows
 // (_add_Bsmat_o! over the three node orderings) have the closed form below in
-// q = C/A, r = D/A, s = A/D.
-FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeom<3> &geo, FxMax &mx)
+// q = C/A, r = D/A, s = A/D.  Returns whether the triangle is longer than T3_LONGEST
+// (STOP: at once, with nothing but that).
+template <bool STOP = false>
+FS_HD bool t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeom<3> &geo, FxMax &mx)
 {
     typedef CompactRows<3, 2> L;
     double J0[3], J1[3], (&e)[3][3] = geo.e;
@@ -294,14 +330,13 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
     cross3(e[2], e[0], e[1]);
     const double q = dot3(J1, e[0]) * ia, r = d * ia, s = a * id;
     const double Jd = a * d, t = in.t;
+    const double far = fmax(fabs(q), fabs(q - 1.0)) * a;
+    const bool elongated = fmax(a * a, fma(far, far, d * d)) > T3_LONGEST * Jd;
+    if (STOP && elongated) return true;
     const double gx0 = -ia, gx1 = ia, gy0 = (q - 1.0) * id, gy1 = -(q * id), gy2 = id;
     geo.g[0][0] = gx0; geo.g[0][1] = gy0;
     geo.g[1][0] = gx1; geo.g[1][1] = gy1;
     geo.g[2][0] = 0.0; geo.g[2][1] = gy2;
-    fx_max(mx.g, gx1);
-    fx_max(mx.g, gy0);
-    fx_max(mx.g, gy1);
-    fx_max(mx.g, gy2);
     // weights: sqrt(t Ae), sqrt(t^3/12 Ae), sqrt(t stab Ae)
     const double sm = sqrt(t * (0.5 * Jd)), sb = sm * t * 0.28867513459481288, ws = sm * t * rsqrt_d(t * t + mc.stab_c * Jd);
     double R2[3][3], m0[3], m1[3];
@@ -316,8 +351,8 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
             const double mu = tx[j] * m0[j] + ty[j] * m1[j];
             ksum += r0 * r0;
             ksum += r1 * r1;
-            fx_max(mx.r, r0);
-            fx_max(mx.r, r1);
+            fx_max(mx.q[j], r0);
+            fx_max(mx.q[j], r1);
             fx_max(mx.u, mu);
             row[3 + 2 * j].d = r0;
             row[4 + 2 * j].d = r1;
@@ -331,8 +366,8 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
         FS_UNROLL
         for (int j = 0; j < 3; j++) {
             const double u = sm * be[j], v = sm * al[j];
-            fx_max(mx.m, u);
-            fx_max(mx.m, v);
+            fx_max(mx.m[j], u);
+            fx_max(mx.m[j], v);
             mr[2 * j].d = u;
             mr[2 * j + 1].d = v;
             tx[j] = -(sb * al[j]);
@@ -371,7 +406,7 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
             const double ty[3] = {f0 * y0[0] + f1 * y1[0], f0 * y0[1] + f1 * y1[1], f0 * y0[2] + f1 * y1[2]};
             FS_UNROLL
             for (int j = 0; j < 3; j++) {
-                fx_max(mx.w, w[j]);
+                fx_max(mx.w[j], w[j]);
                 row[j].d = w[j];
             }
             rotations(row, tx, ty);
@@ -382,7 +417,7 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
         const double ty[3] = {f2 * y1[0], f2 * y1[1], f2 * y1[2]};
         FS_UNROLL
         for (int j = 0; j < 3; j++) {
-            fx_max(mx.w, w[j]);
+            fx_max(mx.w[j], w[j]);
             row[j].d = w[j];
         }
         rotations(row, tx, ty);
@@ -393,6 +428,7 @@ FS_HD void t3_coefs(const ElemIn<3> &in, const MatConst &mc, FxSlots slot, FxGeo
     fx_max(mx.r, sk);
     slot[L::DR].d = sk;
     fx_max_basis(mx, geo);
+    return elongated;
 }
 
 // The membrane rows (MS apart) and the bending and shear rows (from BS, BSS
@@ -412,7 +448,7 @@ FS_HD void expand_slots(FxSlots slot, const FxGeom<NN> &geo, const FxExp &ex, fx
             for (int k = 0; k < 3; k++) e[k][c] = fx_make(geo.e[k][c], 0);
         }
         FS_ROLL
-        for (int k = 0; k < 3; k++) expand_membrane<NN>(slot + MS * k, em, ex.cm);
+        for (int k = 0; k < 3; k++) expand_membrane<NN>(slot + MS * k, em, ex);
     }
     fx g[NN][2];
     TriadFx A[NN];
@@ -420,8 +456,8 @@ FS_HD void expand_slots(FxSlots slot, const FxGeom<NN> &geo, const FxExp &ex, fx
     for (int i = 0; i < NN; i++) {
         A[i] = triad_fx(geo.A[i]);
         triad_axes(A[i], e, t[i]);
-        g[i][0] = fx_make(geo.g[i][0], ex.g);
-        g[i][1] = fx_make(geo.g[i][1], ex.g);
+        g[i][0] = fx_make(geo.g[i][0], ex.g[i]);
+        g[i][1] = fx_make(geo.g[i][1], ex.g[i]);
     }
     FS_ROLL
     for (int k = 0; k < 5; k++) expand_bending<NN>(slot + BS + BSS * k, k >= 3, e[2], t, A, g, ex);
@@ -480,8 +516,6 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
         y[a] = dot3(Xr[a], e[1]);
         geo.g[a][0] = ia * gp[a][0];
         geo.g[a][1] = id * (gp[a][1] - q * gp[a][0]);
-        fx_max(mx.g, geo.g[a][0]);
-        fx_max(mx.g, geo.g[a][1]);
     }
     // weights: sqrt(t Jac), sqrt(t^3/12 Jac), sqrt(t stab Jac)
     const double sm = sqrt(t * (j11 * j22)), sb = sm * t * 0.28867513459481288, ws = sm * ss;
@@ -504,8 +538,8 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
             trace[i] += r0 * r0;
             trace[i] += r1 * r1;
             trace[i] -= p * p;
-            fx_max(mx.r, r0);
-            fx_max(mx.r, r1);
+            fx_max(mx.q[i], r0);
+            fx_max(mx.q[i], r1);
             fx_max(mx.u, mu);
             row[4 + 2 * i].d = r0;
             row[5 + 2 * i].d = r1;
@@ -518,8 +552,8 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
         FS_UNROLL
         for (int i = 0; i < 4; i++) {
             const double u = sm * be[i], v = sm * al[i];
-            fx_max(mx.m, u);
-            fx_max(mx.m, v);
+            fx_max(mx.m[i], u);
+            fx_max(mx.m[i], v);
             mr[2 * i].d = u;
             mr[2 * i + 1].d = v;
             tx[i] = -(sb * al[i]);
@@ -589,7 +623,7 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
         for (int i = 0; i < 4; i++) {
             const int kq = i < 2 ? 0 : 1;
             const double w = g0 * bw[i] + f1 * w1[i];
-            fx_max(mx.w, w);
+            fx_max(mx.w[i], w);
             row[i].d = w;
             tx[i] = g0 * bxx[kq] + f1 * x1[i];
             ty[i] = g0 * bxy[kq] + f1 * y1[i];
@@ -599,7 +633,7 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
         FS_UNROLL
         for (int i = 0; i < 4; i++) {
             const double w = f2 * w1[i];
-            fx_max(mx.w, w);
+            fx_max(mx.w[i], w);
             row[i].d = w;
             tx[i] = f2 * x1[i];
             ty[i] = f2 * y1[i];
@@ -646,81 +680,85 @@ template <int N> FS_HD void fx_load(FxSlots p, fx (&v)[N])
 // on a diagonal block.  top: rows 0..2 of the block into o, bottom: rows 3..5 (on a
 // diagonal block without its first three columns, the transpose of the top's
 // last three).
-template <int NP, int MS, int BS, int BSS, bool DIAG>
-FS_HD void fx_block_top(FxSlots rows, int step, int p, int q, const FxExp &ex, double o[3][6])
+// ex: the exponents, an FxExp or where they lie (node(), em and r of it).
+template <int NP, int MS, int BS, int BSS, bool DIAG, class X>
+FS_HD void fx_block_top(FxSlots rows, int step, int p, int q, const X &ex, double o[3][6])
 {
+    const FxNode a = ex.node(p), b = ex.node(q);
     FxSums m, tt, tr;
     m.zero();
     FS_ROLL
     for (int pt = 0; pt < NP; pt++) {
         FS_UNROLL
         for (int k = 0; k < 3; k++) {
-            fx a[3], b[3];
-            fx_load(rows + pt * step + MS * k + 3 * p, a);
-            fx_load(rows + pt * step + MS * k + 3 * q, b);
-            m.template add<DIAG>(a, b);
+            fx x[3], y[3];
+            fx_load(rows + pt * step + MS * k + 3 * p, x);
+            fx_load(rows + pt * step + MS * k + 3 * q, y);
+            m.template add<DIAG>(x, y);
         }
     }
     FS_UNROLL
     for (int i = 0; i < 3; i++)
         FS_UNROLL
-        for (int j = DIAG ? i : 0; j < 3; j++) o[i][j] = m.value(i, j, ex.m[i] + ex.m[j]);
+        for (int j = DIAG ? i : 0; j < 3; j++) o[i][j] = m.value(i, j, ex.em[i] + ex.em[j] + a.m + b.m);
     tt.zero();
     tr.zero();
     FS_ROLL
     for (int pt = 0; pt < NP; pt++) {
         FS_UNROLL
         for (int k = 0; k < 5; k++) {
-            fx a[3], b[6];
-            fx_load(rows + pt * step + BS + BSS * k + 6 * p, a);
-            fx_load(rows + pt * step + BS + BSS * k + 6 * q, b);
-            tt.template add<DIAG>(a, b);
-            tr.template add<false>(a, b + 3);
+            fx x[3], y[6];
+            fx_load(rows + pt * step + BS + BSS * k + 6 * p, x);
+            fx_load(rows + pt * step + BS + BSS * k + 6 * q, y);
+            tt.template add<DIAG>(x, y);
+            tr.template add<false>(x, y + 3);
         }
     }
     FS_UNROLL
     for (int i = 0; i < 3; i++) {
         FS_UNROLL
         for (int j = DIAG ? i : 0; j < 3; j++) {
-            o[i][j] += tt.value(i, j, 2 * ex.t);
+            o[i][j] += tt.value(i, j, a.t + b.t);
             if (DIAG && j > i) o[j][i] = o[i][j];
         }
         FS_UNROLL
-        for (int j = 0; j < 3; j++) o[i][3 + j] = tr.value(i, j, ex.t + ex.r);
+        for (int j = 0; j < 3; j++) o[i][3 + j] = tr.value(i, j, a.t + b.q);
     }
 }
-template <int NP, int BS, int BSS, bool DIAG>
-FS_HD void fx_block_bottom(FxSlots rows, int step, int p, int q, FxSlots drill, const FxExp &ex,
-                           double o[3][6])
+template <int NP, int BS, int BSS, bool DIAG, class X>
+FS_HD void fx_block_bottom(FxSlots rows, int step, int p, int q, FxSlots drill, const X &ex, double o[3][6])
 {
-    FxSums rt, rr;
+    const FxNode a = ex.node(p), b = ex.node(q);
+    FxSums rt, rr, dd;
     rt.zero();
     rr.zero();
     FS_ROLL
     for (int pt = 0; pt < NP; pt++) {
         FS_UNROLL
         for (int k = 0; k < 5; k++) {
-            fx a[3], b[6];
-            fx_load(rows + pt * step + BS + BSS * k + 6 * p + 3, a);
-            fx_load(rows + pt * step + BS + BSS * k + 6 * q, b);
-            if (!DIAG) rt.template add<false>(a, b);
-            rr.template add<DIAG>(a, b + 3);
+            fx x[3], y[6];
+            fx_load(rows + pt * step + BS + BSS * k + 6 * p + 3, x);
+            fx_load(rows + pt * step + BS + BSS * k + 6 * q, y);
+            if (!DIAG) rt.template add<false>(x, y);
+            rr.template add<DIAG>(x, y + 3);
         }
     }
     if (DIAG) {
         fx d[3];
         fx_load(drill, d);
-        rr.template add<true>(d, d);
+        dd.zero();
+        dd.template add<true>(d, d);
     }
     FS_UNROLL
     for (int i = 0; i < 3; i++) {
         if (!DIAG) {
             FS_UNROLL
-            for (int j = 0; j < 3; j++) o[i][j] = rt.value(i, j, ex.t + ex.r);
+            for (int j = 0; j < 3; j++) o[i][j] = rt.value(i, j, a.q + b.t);
         }
         FS_UNROLL
         for (int j = DIAG ? i : 0; j < 3; j++) {
-            o[i][3 + j] = rr.value(i, j, 2 * ex.r);
+            o[i][3 + j] = rr.value(i, j, a.q + b.q);
+            if (DIAG) o[i][3 + j] += dd.value(i, j, 2 * ex.r);
             if (DIAG && j > i) o[j][3 + i] = o[i][3 + j];
         }
     }

@@ -32,34 +32,46 @@ namespace fs {
 
 static const size_t FX_CHUNK_BYTES = (size_t)1 << 30;  // rows of a chunk
 
-// slots of an element: its rows, then its exponents (m0, m1) (m2, t) (r, done elsewhere)
-constexpr int T3_SLOTS = CompactRows<3, 2>::SIZE + 3;
-constexpr int Q4_SLOTS = Q4Compact::SIZE + 3;
+// slots of an element: its rows, then its exponents (node j: m, t, q, and at the
+// first node whether it is done elsewhere; then em and r)
+constexpr int T3_SLOTS = CompactRows<3, 2>::SIZE + 4;
+constexpr int Q4_SLOTS = Q4Compact::SIZE + 5;
 
 __device__ __forceinline__ FxSlots fx_slots(FxSlot *rows, int nslots, int64_t e)
 {
     return FxSlots{rows + (e / FX_GROUP) * (FX_GROUP * nslots) + e % FX_GROUP};
 }
-__device__ __forceinline__ void put_exponents(FxSlots x, const FxExp &ex, bool redo)
+template <int NN> __device__ __forceinline__ void put_exponents(FxSlots x, const FxExp &ex, bool redo)
 {
-    x[0].x = fx{ex.m[0], ex.m[1]};
-    x[1].x = fx{ex.m[2], ex.t};
-    x[2].x = fx{ex.r, redo ? 1 : 0};
+    auto put = [](FxSlot &o, int a, int b, int c, int d) {
+        o.x = fx{(int)((unsigned)(a & 0xffff) | (unsigned)b << 16), (int)((unsigned)(c & 0xffff) | (unsigned)d << 16)};
+    };
+#pragma unroll
+    for (int j = 0; j < NN; j++) put(x[j], ex.m[j], ex.t[j], ex.q[j], j == 0 && redo);
+    put(x[NN], ex.em[0], ex.em[1], ex.em[2], ex.r);
 }
-__device__ __forceinline__ bool get_exponents(FxSlots x, FxExp &ex)
-{
-    const fx a = x[0].x, b = x[1].x, c = x[2].x;
-    ex.m[0] = a.h;
-    ex.m[1] = a.l;
-    ex.m[2] = b.h;
-    ex.t = b.l;
-    ex.r = c.h;
-    return c.l != 0;
-}
+// the exponents of an element where they lie
+template <int NN> struct StoredExp {
+    FxSlots x;
+    int em[3], r;
+    __device__ __forceinline__ explicit StoredExp(FxSlots slots) : x(slots)
+    {
+        const FxSlot v = x[NN];
+#pragma unroll
+        for (int c = 0; c < 3; c++) em[c] = v.s[c];
+        r = v.s[3];
+    }
+    __device__ __forceinline__ bool redo() const { return x[0].s[3] != 0; }
+    __device__ __forceinline__ FxNode node(int j) const
+    {
+        const FxSlot v = x[j];
+        return FxNode{v.s[0], v.s[1], v.s[2]};
+    }
+};
 
 // elements e0 .. e0 + n of a chunk; an element whose coefficients do not suit
 // the fixed point (not finite, or next to a double's limits: a degenerate
-// one) is marked in `redo` for the double kernel
+// one; a triangle longer than T3_LONGEST) is marked in `redo` for the double kernel
 __global__ void __launch_bounds__(128, 3) k_t3_rows(const MeshDev m, const MatConst mc, int64_t e0, int64_t n, FxSlot *rows,
                                                  uint8_t *redo, int *status)
 {
@@ -70,12 +82,11 @@ __global__ void __launch_bounds__(128, 3) k_t3_rows(const MeshDev m, const MatCo
     load_elem<3>(m, e0 + e, in);
     FxGeom<3> geo;
     FxMax mx;
-    t3_coefs(in, mc, slot, geo, mx);
-    const bool bad = !mx.usable();
+    const bool bad = t3_coefs<true>(in, mc, slot, geo, mx) || !mx.usable();
     if (bad) atomicOr(status, DEV_REDO);
     redo[e0 + e] = bad;
     FxExp ex = fx_exponents(mx, 0);
-    put_exponents(slot + CompactRows<3, 2>::SIZE, ex, bad);
+    put_exponents<3>(slot + CompactRows<3, 2>::SIZE, ex, bad);
     if (!bad) t3_expand(slot, geo, in.valid, ex);
 }
 
@@ -97,8 +108,8 @@ __global__ void __launch_bounds__(96, 4) k_t3_gram(const MeshDev m, int64_t e0, 
     }
     if (e >= n) return;
     const FxSlots slot{fx_smem + (threadIdx.x & 31)};
-    FxExp ex;
-    if (get_exponents(slot + L::SIZE, ex)) return;
+    const StoredExp<3> ex(slot + L::SIZE);
+    if (ex.redo()) return;
     double *out = ke + r * (6 * 36);
     // block (w, w)
     {
@@ -205,23 +216,28 @@ __global__ void __launch_bounds__(128, 3) k_q4_rows(const MeshDev m, const MatCo
         dr[c] = sk * sg.nrm[qp][c];
         fx_max(mx.r, dr[c]);
     }
-    auto over_points = [&](uint32_t &v) {
-        v = max(v, __shfl_xor_sync(mask, v, 1));
-        v = max(v, __shfl_xor_sync(mask, v, 2));
+    // maxima over the points, two at a time by their exponent fields
+    auto over_points = [&](uint32_t &a, uint32_t &b) {
+        uint32_t v = __byte_perm(a >> 20, b >> 20, 0x5410);
+        v = __vmaxu2(v, __shfl_xor_sync(mask, v, 1));
+        v = __vmaxu2(v, __shfl_xor_sync(mask, v, 2));
+        a = v << 20;
+        b = (v >> 16) << 20;
     };
-    over_points(mx.m);
-    over_points(mx.w);
-    over_points(mx.r);
-    over_points(mx.u);
-    over_points(mx.g);
 #pragma unroll
-    for (int c = 0; c < 3; c++) over_points(mx.e[c]);
+    for (int k = 0; k < 4; k++) {
+        over_points(mx.m[k], mx.w[k]);
+        over_points(mx.q[k], mx.g[k]);
+    }
+    over_points(mx.r, mx.u);
+    over_points(mx.e[0], mx.e[1]);
+    over_points(mx.e[2], mx.e[2]);
     bad = __any_sync(mask, bad || !mx.usable());
     const FxExp ex = fx_exponents(mx, 1);
     if (qp == 0) {
         if (bad) atomicOr(status, DEV_REDO);
         redo[r] = bad;
-        put_exponents(es + L::SIZE, ex, bad);
+        put_exponents<4>(es + L::SIZE, ex, bad);
     }
     if (bad) return;
     fx t[4][3][3];
@@ -237,8 +253,8 @@ __global__ void __launch_bounds__(128, 3) k_q4_gram(const MeshDev m, int64_t e0,
     const int64_t e = (int64_t)blockIdx.x * FX_GROUP + (threadIdx.x & 31), r = e0 + e;
     if (e >= n) return;
     const FxSlots slot = fx_slots(rows, Q4_SLOTS, e);
-    FxExp ex;
-    if (get_exponents(slot + L::SIZE, ex)) return;
+    const StoredExp<4> ex(slot + L::SIZE);
+    if (ex.redo()) return;
     const unsigned swapped = swapped_blocks<4>(m.conn + r * 4);
     double *out = ke + r * (10 * 36);
     // every warp a diagonal block, then three of the twelve halves of the
