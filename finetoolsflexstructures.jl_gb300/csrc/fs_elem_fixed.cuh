@@ -24,8 +24,8 @@
 // elongation (longest edge squared over twice the area): at most 1.1 up to 32, 1.4
 // from 32 to 64, 2.2 from 64 to 128 (a rotation's shear energy on an axis-aligned
 // plate); with one exponent for all nodes 1.7 from 4 to 8, 2.7 from 16 to 32.
-// Quadrilaterals: 1.9 at most at any elongation, and the matrix is nearer than
-// double's (16 to 1: 0.4 of its error, 256 to 1: 0.002), whose own rows lose more;
+// Quadrilaterals: 1.4 at most but for strongly sheared ones (1.6), and the matrix is
+// nearer than double's (16 to 1: 0.4 of its error, 256 to 1: 0.002), whose own rows lose more;
 // none is left.  Exponents by node cost 3 % (elements, triangles, 700 x 700: 1.53 and
 // 1.58 ms, quads, 360 x 360: 1.54 and 1.59); a plate of nothing but long triangles takes
 // 5.0 ms instead of 2.05 (4.8 when all was double).
@@ -601,7 +601,10 @@ FS_HD int q4_coefs(const double Xr[4][3], const double nrm[4][3], const bool val
         const double ax = x01 * sp + x23 * sm1, ay = y01 * sp + y23 * sm1;
         const double bx = x03 * rp - x12 * rm, by = y03 * rp - y12 * rm;
         const double LA = sqrt(ax * ax + ay * ay), LB2 = bx * bx + by * by, B2 = j12 * j12 + j22 * j22;
-        const double d32 = ia * id * 0.03125, kb = LB2 * rsqrt_d(LB2 * B2) * d32;  // LB / B / (32 det)
+        // 1 / (32 det), the reciprocal with one Newton step: a factor of all shear entries
+        // (their energies 1.7 times as far off as in double without, 1.3 with; elements,
+        // quads 360 x 360: 1.59 and 1.62 ms)
+        const double rd = ia * id, d32 = fma(fma(-j11 * j22, rd, 1.0), rd, rd) * 0.03125, kb = LB2 * rsqrt_d(LB2 * B2) * d32;  // LB / B / (32 det)
         const double q0 = j22 * kb, q1 = -(j12 * kb), p1 = -(LA * d32);
         const double f0 = ws * mc.Lt[lp(0, 0)], f1 = ws * mc.Lt[lp(1, 0)], f2 = ws * mc.Lt[lp(1, 1)];
         // node-wise factors of the two terms (w, thx, thy)

@@ -1,4 +1,4 @@
-// Test-only host build: element matrices of triangles in the FS_FP64 fixed point
+// Test-only host build: element matrices in the FS_FP64 fixed point
 // (csrc/fs_elem_fixed.cuh) and in double (csrc/fs_elem_math.cuh), less the same in
 // long double (wide_elem_math.h, the latter header with every double widened).
 // Not part of the product.
@@ -13,11 +13,11 @@
 
 using namespace fs;
 
-template <class E> static E element(const double *X, const double *nrm, double t)
+template <class E, int NN = 3> static E element(const double *X, const double *nrm, double t)
 {
     E in;
     memset(&in, 0, sizeof in);
-    for (int a = 0; a < 3; a++) {
+    for (int a = 0; a < NN; a++) {
         for (int c = 0; c < 3; c++) {
             in.X[a][c] = X[3 * a + c];
             in.nrm[a][c] = nrm[3 * a + c];
@@ -26,6 +26,60 @@ template <class E> static E element(const double *X, const double *nrm, double t
     }
     in.t = t;
     return in;
+}
+
+// node blocks from expanded rows
+template <int NP, int NN, int MS, int BS, int BSS, int DR>
+static void blocks(FxSlots rows, int step, const FxExp &ex, double *K)
+{
+    for (int p = 0; p < NN; p++)
+        for (int q = 0; q < NN; q++) {
+            double o[3][6], b[3][6];
+            if (p == q) {
+                fx_block_top<NP, MS, BS, BSS, true>(rows, step, p, q, ex, o);
+                fx_block_bottom<NP, BS, BSS, true>(rows, step, p, q, rows + (DR + 3 * p), ex, b);
+                for (int i = 0; i < 3; i++)
+                    for (int j = 0; j < 3; j++) b[i][j] = o[j][3 + i];
+            } else {
+                fx_block_top<NP, MS, BS, BSS, false>(rows, step, p, q, ex, o);
+                fx_block_bottom<NP, BS, BSS, false>(rows, step, p, q, rows, ex, b);
+            }
+            for (int i = 0; i < 3; i++)
+                for (int j = 0; j < 6; j++) {
+                    K[(6 * p + i) * 6 * NN + 6 * q + j] = o[i][j];
+                    K[(6 * p + 3 + i) * 6 * NN + 6 * q + j] = b[i][j];
+                }
+        }
+}
+
+// the outputs of one element: the long double matrix (rounded) and the differences
+// of the fixed point's, F, and of the double rows' from it
+static void compare(int nd, int nrows, const double *F, const double *rows, const long double *wide, double *K,
+                    double *dfixed, double *ddouble)
+{
+    for (int i = 0; i < nd; i++)
+        for (int j = 0; j < nd; j++) {
+            double d = 0;
+            long double s = 0;
+            for (int r = 0; r < nrows; r++) {
+                d = fma(rows[nd * r + i], rows[nd * r + j], d);
+                s += wide[nd * r + i] * wide[nd * r + j];
+            }
+            K[nd * i + j] = (double)s;
+            dfixed[nd * i + j] = (double)(F[nd * i + j] - s);
+            ddouble[nd * i + j] = (double)(d - s);
+        }
+}
+
+static int constants(const fs_shell_params &p, MatConst &mc, fsl::MatConst &ml)
+{
+    if (prepare_matconst(p, mc)) return 1;
+    memset(&ml, 0, sizeof ml);
+    for (int i = 0; i < 6; i++) ml.Lps[i] = mc.Lps[i];
+    for (int i = 0; i < 3; i++) ml.Lt[i] = mc.Lt[i];
+    ml.stab_c = mc.stab_c;
+    ml.drill_scale = mc.drill_scale;
+    return 0;
 }
 
 extern "C" {
@@ -37,20 +91,15 @@ int stretched_triangles(int64_t n, const double *X, const double *nrm, const dou
                         double *K, double *dfixed, double *ddouble, uint8_t *elongated)
 {
     MatConst mc;
-    if (prepare_matconst(*p, mc)) return 1;
     fsl::MatConst ml;
-    memset(&ml, 0, sizeof ml);
-    for (int i = 0; i < 6; i++) ml.Lps[i] = mc.Lps[i];
-    for (int i = 0; i < 3; i++) ml.Lt[i] = mc.Lt[i];
-    ml.stab_c = mc.stab_c;
-    ml.drill_scale = mc.drill_scale;
+    if (constants(*p, mc, ml)) return 1;
     typedef CompactRows<3, 2> L;
     static FxSlot mem[(L::SIZE + 1) * FX_GROUP];
     const FxSlots slot{mem};
     for (int64_t e = 0; e < n; e++) {
         const ElemIn<3> in = element<ElemIn<3>>(X + 9 * e, nrm + 9 * e, t[e]);
         const fsl::ElemIn<3> il = element<fsl::ElemIn<3>>(X + 9 * e, nrm + 9 * e, t[e]);
-        double rows[11 * 18], F[18][18];
+        double rows[11 * 18], F[324];
         long double wide[11 * 18];
         t3_rows<double, false, false>(in, mc, nullptr, rows, 18);
         fsl::t3_rows<long double, false, false>(il, ml, nullptr, wide, 18);
@@ -60,37 +109,56 @@ int stretched_triangles(int64_t n, const double *X, const double *nrm, const dou
         if (!mx.usable()) return 2;
         const FxExp ex = fx_exponents(mx, 0);
         t3_expand(slot, geo, in.valid, ex);
-        for (int p = 0; p < 3; p++)
-            for (int q = 0; q < 3; q++) {
-                double o[3][6], b[3][6];
-                if (p == q) {
-                    fx_block_top<1, L::MS, L::BS, L::BSS, true>(slot, 0, p, q, ex, o);
-                    fx_block_bottom<1, L::BS, L::BSS, true>(slot, 0, p, q, slot + (L::DR + 3 * p), ex, b);
-                    for (int i = 0; i < 3; i++)
-                        for (int j = 0; j < 3; j++) b[i][j] = o[j][3 + i];
-                } else {
-                    fx_block_top<1, L::MS, L::BS, L::BSS, false>(slot, 0, p, q, ex, o);
-                    fx_block_bottom<1, L::BS, L::BSS, false>(slot, 0, p, q, slot, ex, b);
-                }
-                for (int i = 0; i < 3; i++)
-                    for (int j = 0; j < 6; j++) {
-                        F[6 * p + i][6 * q + j] = o[i][j];
-                        F[6 * p + 3 + i][6 * q + j] = b[i][j];
-                    }
-            }
-        for (int i = 0; i < 18; i++)
-            for (int j = 0; j < 18; j++) {
-                double d = 0;
-                long double s = 0;
-                for (int r = 0; r < 11; r++) {
-                    d = fma(rows[18 * r + i], rows[18 * r + j], d);
-                    s += wide[18 * r + i] * wide[18 * r + j];
-                }
-                const int64_t at = 324 * e + 18 * i + j;
-                K[at] = (double)s;
-                dfixed[at] = (double)(F[i][j] - s);
-                ddouble[at] = (double)(d - s);
-            }
+        blocks<1, 3, L::MS, L::BS, L::BSS, L::DR>(slot, 0, ex, F);
+        compare(18, 11, F, rows, wide, K + 324 * e, dfixed + 324 * e, ddouble + 324 * e);
+    }
+    return 0;
+}
+
+// the same of n quadrilaterals (4 x 3 each, 24 x 24)
+int stretched_quads(int64_t n, const double *X, const double *nrm, const double *t, const fs_shell_params *p, double *K,
+                    double *dfixed, double *ddouble)
+{
+    MatConst mc;
+    fsl::MatConst ml;
+    if (constants(*p, mc, ml)) return 1;
+    typedef Q4Compact L;
+    static FxSlot mem[(L::SIZE + 1) * FX_GROUP];
+    const FxSlots slot{mem};
+    for (int64_t e = 0; e < n; e++) {
+        const ElemIn<4> in = element<ElemIn<4>, 4>(X + 12 * e, nrm + 12 * e, t[e]);
+        const fsl::ElemIn<4> il = element<fsl::ElemIn<4>, 4>(X + 12 * e, nrm + 12 * e, t[e]);
+        Q4Elem qe;
+        fsl::Q4Elem ql;
+        q4_prepare(in, in.t, mc.stab_c, qe);
+        fsl::q4_prepare(il, il.t, ml.stab_c, ql);
+        double rows[36 * 24], F[576], td[4] = {0, 0, 0, 0}, tp[4], tr[4] = {0, 0, 0, 0}, rn[4], sum = 0;
+        long double wide[36 * 24], tl[4] = {0, 0, 0, 0}, tq[4];
+        FxGeom<4> geo[4];
+        FxMax mx;
+        for (int k = 0; k < 4; k++) rn[k] = 1.0 / sqrt(dot3(in.nrm[k], in.nrm[k]));
+        for (int j = 0; j < 4; j++) {
+            if (q4_coefs(qe.Xr, in.nrm, in.valid, rn, in.t, sqrt(qe.stab), j, mc, slot + j * L::GP, geo[j], mx, tp)) return 2;
+            for (int k = 0; k < 4; k++) tr[k] += tp[k];
+            q4_point_rows<double, false>(in, qe, j, mc, nullptr, rows + j * 8 * 24, 24, tp);
+            for (int k = 0; k < 4; k++) td[k] += tp[k];
+            fsl::q4_point_rows<long double, false>(il, ql, j, ml, nullptr, wide + j * 8 * 24, 24, tq);
+            for (int k = 0; k < 4; k++) tl[k] += tq[k];
+        }
+        q4_drill_rows<double>(in, td, mc.drill_scale, rows + 32 * 24, 24);
+        fsl::q4_drill_rows<long double>(il, tl, ml.drill_scale, wide + 32 * 24, 24);
+        for (int k = 0; k < 4; k++) sum += tr[k] > 0.0 ? tr[k] / 2 : 0.0;
+        const double sk = sqrt(sum / 4 * mc.drill_scale);
+        for (int k = 0; k < 12; k++) fx_max(mx.r, sk * in.nrm[k / 3][k % 3]);
+        if (!mx.usable()) return 3;
+        const FxExp ex = fx_exponents(mx, 1);
+        for (int j = 0; j < 4; j++) {
+            fx ax[4][3][3];
+            expand_slots<4, L::MS, L::BS, L::BSS>(slot + j * L::GP, geo[j], ex, ax);
+        }
+        for (int k = 0; k < 12; k++) slot[L::DR + k].x = fx_make(sk * in.nrm[k / 3][k % 3], ex.r);
+        blocks<4, 4, L::MS, L::BS, L::BSS, L::DR>(slot, L::GP, ex, F);
+        compare(24, 36, F, rows, wide, K + 576 * e, dfixed + 576 * e, ddouble + 576 * e);
     }
     return 0;
 }
