@@ -4,8 +4,8 @@
 #pragma once
 
 #include "fs_comp_sum.cuh"
-#include "fs_fixed.cuh"
 #include "fs_internal.cuh"
+#include "fs_elem_fixed.cuh"
 
 namespace fs {
 
@@ -336,93 +336,18 @@ __device__ __forceinline__ void write_blocks_compact(const R *rows, unsigned swa
         });
 }
 
-// Double rows of a layered element multiplied in fixed point (FS_FP64): the
-// values of each of a node's six dofs, over all rows and nodes, share an exponent,
-// so that a row entry is kept to 2^-58 of its dof's largest, and the products
-// are exact sums of integers (fs_fixed.cuh), rounded once.  In double the
-// products are half of the kernel's double operations (T3FFComp, 257 x 190: 0.65 ms,
-// now 0.55; Q4RSComp, 512 x 512: 10.6 and 8.1).
-struct DofMax {
-    uint32_t m[6] = {0, 0, 0, 0, 0, 0};
-    // one value per dof of N nodes
-    template <int N> __device__ __forceinline__ void row(const double *r)
-    {
-#pragma unroll
-        for (int k = 0; k < 6 * N; k++) fx_max(m[k % 6], r[k]);
-    }
-    __device__ __forceinline__ void rotations(const double *r)
-    {
-#pragma unroll
-        for (int k = 0; k < 3; k++) fx_max(m[3 + k], r[k]);
-    }
-    __device__ __forceinline__ bool usable() const
-    {
-        bool ok = true;
-#pragma unroll
-        for (int k = 0; k < 6; k++) ok = ok && fx_usable(m[k]);
-        return ok;
-    }
-    // spare: bits kept free for long sums
-    __device__ __forceinline__ void exponents(int (&E)[6], int spare) const
-    {
-#pragma unroll
-        for (int k = 0; k < 6; k++) E[k] = fx_group(m[k]) + spare;
-    }
-};
-// a double in shared memory replaced by its fixed-point number
-__device__ __forceinline__ void to_fixed(double *p, int E) { *reinterpret_cast<fx *>(p) = fx_make(*p, E); }
-
-// Rows i0 .. i0 + 2 (i0 = 0 or 3) of node block (a, b) from NR rows (stride RS) in
-// fixed point; UPPER: of a diagonal block (i0 = I0), its entries (i, j), j >= i, with
-// the drilling row of the node (dr: its rotations)
-template <int NR, int RS, bool UPPER, int I0>
-__device__ __forceinline__ void fixed_rows(const double *rows, const double *dr, int a, int b, const int (&E)[6],
-                                           double (&o)[3][6], int i0 = I0)
-{
-    FxSum s[3][6];
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 6; j++) s[i][j] = FxSum{0, 0};
-    const fx *ra = reinterpret_cast<const fx *>(rows) + 6 * a + i0, *rb = reinterpret_cast<const fx *>(rows) + 6 * b;
-#pragma unroll 8
-    for (int r = 0; r < NR; r++) {
-        fx x[3], y[6];
-#pragma unroll
-        for (int i = 0; i < 3; i++) x[i] = ra[r * RS + i];
-#pragma unroll
-        for (int j = UPPER ? I0 : 0; j < 6; j++) y[j] = rb[r * RS + j];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = UPPER ? I0 + i : 0; j < 6; j++) fx_mac(s[i][j], x[i], y[j]);
-    }
-    if constexpr (UPPER && I0 == 3) {
-        fx d[3];
-#pragma unroll
-        for (int i = 0; i < 3; i++) d[i] = reinterpret_cast<const fx *>(dr)[i];
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = i; j < 3; j++) fx_mac(s[i][3 + j], d[i], d[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = UPPER ? I0 + i : 0; j < 6; j++) o[i][j] = fx_double(s[i][j], (i0 ? E[3 + i] : E[i]) + E[j]);
-}
-// a diagonal block whole
+// a diagonal block of a layered element from its fixed-point rows, whole
 template <int NR, int RS>
-__device__ __forceinline__ void fixed_diagonal(const double *rows, const double *dr, int a, const int (&E)[6], double *out)
+__device__ __forceinline__ void fixed_diagonal(const double *rows, const double *dr, int a, DofExp E, double *out)
 {
     double t[3][6], u[3][6];
-    fixed_rows<NR, RS, true, 0>(rows, dr, a, a, E, t);
+    fixed_rows<NR, RS, true, 0>(rows, dr, a, a, E, E, t);
 #pragma unroll
     for (int i = 1; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < i; j++) t[i][j] = t[j][i];
     store_rows<double, 3>(out, t);
-    fixed_rows<NR, RS, true, 3>(rows, dr, a, a, E, u);
+    fixed_rows<NR, RS, true, 3>(rows, dr, a, a, E, E, u);
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
@@ -432,11 +357,17 @@ __device__ __forceinline__ void fixed_diagonal(const double *rows, const double 
 
 // Upper node blocks of a layered element from its fixed-point rows
 template <int NN, int NR>
-__device__ __forceinline__ void write_blocks_fixed(const double *rows, const int (&E)[6], unsigned swapped, double *out)
+__device__ __forceinline__ void write_blocks_fixed(const double *rows, const DofExp (&E)[NN], unsigned swapped, double *out)
 {
     typedef LayeredRows<NN, NR> L;
+    auto of = [&](int a) {
+        DofExp e = E[0];
+#pragma unroll
+        for (int k = 1; k < NN; k++) e = a == k ? E[k] : e;
+        return e;
+    };
 #pragma unroll 1
-    for (int a = 0; a < NN; a++) fixed_diagonal<NR, L::RS>(rows, rows + L::DR + 3 * a, a, E, out + ub(a, a, NN) * 36);
+    for (int a = 0; a < NN; a++) fixed_diagonal<NR, L::RS>(rows, rows + L::DR + 3 * a, a, of(a), out + ub(a, a, NN) * 36);
 #pragma unroll 1
     for (int a = 0; a < NN; a++)
 #pragma unroll 1
@@ -446,7 +377,7 @@ __device__ __forceinline__ void write_blocks_fixed(const double *rows, const int
 #pragma unroll 1
             for (int i0 = 0; i0 < 6; i0 += 3) {
                 double o[3][6];
-                fixed_rows<NR, L::RS, false, 0>(rows, rows, p, q, E, o, i0);
+                fixed_rows<NR, L::RS, false, 0>(rows, rows, p, q, of(p), of(q), o, i0);
                 store_rows<double, 3>(out + ub(a, b, NN) * 36 + 6 * i0, o);
             }
         }

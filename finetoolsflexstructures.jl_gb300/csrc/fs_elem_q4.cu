@@ -180,40 +180,53 @@ __global__ void __launch_bounds__(128, 2)
     __syncwarp();
     if constexpr (FIXED) {
         // the element's exponents, then its rows to fixed point, a fourth a lane
-        DofMax mx;
+        DofMax<4> mx;
+        mx.zero();
         if (active) {
-            for (int k = 8 * qp; k < 8 * qp + 8; k++) mx.template row<4>(rows + k * ND);
-            mx.rotations(rows + DR + 3 * qp);
-        }
+            for (int k = 8 * qp; k < 8 * qp + 8; k++) mx.row(rows + k * ND);
 #pragma unroll
-        for (int k = 0; k < 6; k++) {
-            mx.m[k] = max(mx.m[k], __shfl_xor_sync(0xffffffffu, mx.m[k], 1));
-            mx.m[k] = max(mx.m[k], __shfl_xor_sync(0xffffffffu, mx.m[k], 2));
+            for (int k = 0; k < 12; k++)
+                if (k / 3 == qp) fx_max(mx.m[k / 3][3 + k % 3], rows[DR + k]);
+        }
+        // over the lanes, two at a time by their exponent fields
+#pragma unroll
+        for (int k = 0; k < 24; k += 2) {
+            uint32_t v = __byte_perm(mx.m[k / 6][k % 6] >> 20, mx.m[k / 6][k % 6 + 1] >> 20, 0x5410);
+            v = __vmaxu2(v, __shfl_xor_sync(0xffffffffu, v, 1));
+            v = __vmaxu2(v, __shfl_xor_sync(0xffffffffu, v, 2));
+            mx.m[k / 6][k % 6] = v << 20;
+            mx.m[k / 6][k % 6 + 1] = (v >> 16) << 20;
         }
         const bool fixed = active && mx.usable();
-        int E[6];
-        mx.exponents(E, 1);
+        DofExp E[4];
+#pragma unroll
+        for (int a = 0; a < 4; a++) E[a] = mx.exponents(a, 1);
+        auto of = [&](int a) { return a == 0 ? E[0] : a == 1 ? E[1] : a == 2 ? E[2] : E[3]; };
         if (fixed) {
+#pragma unroll
+            for (int a = 0; a < 4; a++)
 #pragma unroll 1
-            for (int k = 32 * qp; k < 32 * qp + 32; k++)
+                for (int k = 8 * qp; k < 8 * qp + 8; k++)
 #pragma unroll
-                for (int q = 0; q < 6; q++) to_fixed(rows + 6 * k + q, E[q]);
+                    for (int q = 0; q < 6; q++) to_fixed(rows + ND * k + 6 * a + q, dof_exp(E[a], q));
+            const DofExp e = of(qp);
 #pragma unroll
-            for (int k = 0; k < 3; k++) to_fixed(rows + DR + 3 * qp + k, E[3 + k]);
+            for (int k = 0; k < 3; k++) to_fixed(rows + DR + 3 * qp + k, dof_exp(e, 3 + k));
         }
         __syncwarp();
         if (fixed) {
             double *o = ke + r * (10 * 36);
             const unsigned swapped = swapped_blocks<4>(m.conn + r * 4);
-            fixed_diagonal<32, ND>(rows, rows + DR + 3 * qp, qp, E, o + ub(qp, qp, 4) * 36);
+            fixed_diagonal<32, ND>(rows, rows + DR + 3 * qp, qp, of(qp), o + ub(qp, qp, 4) * 36);
 #pragma unroll 1
             for (int t = 0; t < 3; t++) {
                 const int u = qp + 4 * t, ob = u < 6 ? u : u - 6, i0 = u < 6 ? 0 : 3;
                 const int a0 = ob < 3 ? 0 : (ob < 5 ? 1 : 2);
                 const int b0 = ob < 3 ? ob + 1 : (ob < 5 ? ob - 1 : 3);
                 const bool sw = (swapped >> (4 * a0 + b0)) & 1u;
+                const int p = sw ? b0 : a0, q = sw ? a0 : b0;
                 double v[3][6];
-                fixed_rows<32, ND, false, 0>(rows, rows, sw ? b0 : a0, sw ? a0 : b0, E, v, i0);
+                fixed_rows<32, ND, false, 0>(rows, rows, p, q, of(p), of(q), v, i0);
                 store_rows<double, 3>(o + ub(a0, b0, 4) * 36 + 6 * i0, v);
             }
             return;

@@ -43,18 +43,23 @@ __global__ void __launch_bounds__(128, (T3MinBlocks<R, COMP, AVGK, S>::value))
     const unsigned swapped = swapped_blocks<3>(m.conn + r * 3);
     if constexpr (FIXED) {
         typedef LayeredRows<3, 6 + NS> L;
-        DofMax mx;
-        for (int k = 0; k < 6 + NS; k++) mx.template row<3>(rows + k * ND);
-        for (int k = 0; k < 3; k++) mx.rotations(rows + L::DR + 3 * k);
+        DofMax<3> mx;
+        mx.zero();
+        for (int k = 0; k < 6 + NS; k++) mx.row(rows + k * ND);
+#pragma unroll
+        for (int k = 0; k < 9; k++) fx_max(mx.m[k / 3][3 + k % 3], rows[L::DR + k]);
         if (mx.usable()) {
-            int E[6];
-            mx.exponents(E, 0);
+            DofExp E[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                E[a] = mx.exponents(a, 0);
 #pragma unroll 1
-            for (int k = 0; k < 3 * (6 + NS); k++)
+                for (int k = 0; k < 6 + NS; k++)
 #pragma unroll
-                for (int q = 0; q < 6; q++) to_fixed(rows + 6 * k + q, E[q]);
+                    for (int q = 0; q < 6; q++) to_fixed(rows + ND * k + 6 * a + q, dof_exp(E[a], q));
 #pragma unroll
-            for (int k = 0; k < 9; k++) to_fixed(rows + L::DR + k, E[3 + k % 3]);
+                for (int q = 0; q < 3; q++) to_fixed(rows + L::DR + 3 * a + q, dof_exp(E[a], 3 + q));
+            }
             write_blocks_fixed<3, 6 + NS>(rows, E, swapped, ke + r * (6 * 36));
             return;
         }

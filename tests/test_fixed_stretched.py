@@ -36,7 +36,7 @@ def lib(tmp_path_factory):
         src = re.sub(r"(?<![\w.])%s\(" % f, f + "l(", src)
     (d / "wide_elem_math.h").write_text(src)
     so = str(d / "libstretch.so")
-    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-I", CSRC, "-I", str(d),
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-fno-strict-aliasing", "-I", CSRC, "-I", str(d),
                     "-I", os.path.join(os.path.dirname(HERE), "include"), "-o", so,
                     os.path.join(HERE, "hostcheck", "stretchcheck.cpp")], check=True)
     return ctypes.CDLL(so)
