@@ -151,6 +151,7 @@ static BeamDev beam_dev(fs_ctx *c)
 
 int launch_beam_elements(fs_ctx *c, int which, int mass_type)
 {
+    c->fx_marks.launch();
     MeshDev &m = c->mesh;
     const size_t bytes = (size_t)m.nelem * 108 * sizeof(double);
     if (bytes > c->ke_bytes || !c->ke) {

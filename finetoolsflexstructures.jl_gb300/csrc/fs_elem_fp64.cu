@@ -26,7 +26,6 @@
 
 #include "fs_elem_common.cuh"
 #include "fs_elem_fixed.cuh"
-#include "fs_fp64_rows.h"
 
 namespace fs {
 
@@ -328,6 +327,7 @@ int run_fp64(fs_ctx *c, double *ke)
     int epb = c->tune.elem_epb;
     if (t3 && epb != 32 && epb != 64) epb = 128;
     if (!t3 && epb != 8 && epb != 16) epb = 32;
+    c->fx_marks.made();
     for (int64_t e0 = 0; e0 < m.nelem; e0 += chunk) {
         const int64_t n = std::min(chunk, m.nelem - e0);
         const unsigned groups = (unsigned)((n + FX_GROUP - 1) / FX_GROUP);
@@ -349,8 +349,9 @@ int run_fp64(fs_ctx *c, double *ke)
 int read_element_status(fs_ctx *c, int precision, void *ke, double *vals, int *bits)
 {
     FS_TRY(read_status(c, bits));
-    if (!(*bits & DEV_REDO)) return FS_OK;
-    const int first = *bits & ~DEV_REDO;
+    const bool redo = c->fx_marks.redo(*bits & DEV_REDO);
+    const int first = *bits &= ~DEV_REDO;
+    if (!redo) return FS_OK;
     FS_TRY(c->mesh.nen == 3 ? redo_t3(c, (double *)ke, (const uint8_t *)c->fx_rows) : redo_q4(c, (double *)ke, (const uint8_t *)c->fx_rows));
     if (vals) FS_TRY(launch_gather_from(c, precision, ke, vals));
     FS_TRY(read_status(c, bits));

@@ -1,6 +1,6 @@
-// Sizes of the FS_FP64 elements' row buffer (fs_elem_fp64.cu): a byte of mark per
-// element, then the rows of a chunk of elements, in groups.  Host code without
-// CUDA, so that it can be tested with made-up capacities.
+// The FS_FP64 elements' row buffer (fs_elem_fp64.cu): a byte of mark per element,
+// then the rows of a chunk of elements, in groups.  Host code without CUDA, so that
+// it can be tested with made-up capacities.
 #pragma once
 #include <stddef.h>
 
@@ -32,5 +32,21 @@ int fx_reserve(size_t cap, size_t &asked, size_t marks, size_t want, size_t grou
         if (want == least) return ok;
     }
 }
+
+// Whether the marks of the elements to do in double are those of the last element
+// kernels.  The device's flag that there are any stays until it is read, so one
+// that is left by a call which failed in between must not have a later call's
+// matrices (other elements, another precision) done over.
+struct FxMarks {
+    bool fresh = false;
+    void launch() { fresh = false; }  // element kernels are about to run
+    void made() { fresh = true; }     // they write marks
+    bool redo(bool flagged)           // the flag was read: are there elements to do over?
+    {
+        const bool r = fresh && flagged;
+        fresh = false;
+        return r;
+    }
+};
 
 }  // namespace fs

@@ -9,6 +9,7 @@
 #include "../../include/flexshell.h"
 #include "fs_elem_math.cuh"
 #include "fs_beam_math.cuh"
+#include "fs_fp64_rows.h"
 
 namespace fs {
 
@@ -145,6 +146,7 @@ struct fs_ctx {
     // FS_FP64: rows of a chunk of elements, and the elements to do in double
     void *fx_rows = nullptr;
     size_t cap_fx_rows = 0, fx_asked = 0;
+    fs::FxMarks fx_marks;
     bool drops_zeros = false;  // during an assembly that drops exact zeros
     // current matrix; mat_kind 0 a stiffness (shell or beam), 1 a mass, 2
     // another beam matrix

@@ -44,6 +44,7 @@ size_t entry_bytes(int precision) { return precision == FS_MIXED ? 4 : 8; }
 
 int launch_elements(fs_ctx *c, int precision)
 {
+    c->fx_marks.launch();
     MeshDev &m = c->mesh;
     size_t bytes = (size_t)m.nelem * n_upper_blocks(m.nen) * 36 * entry_bytes(precision);
     if (bytes > c->ke_bytes) {
@@ -321,6 +322,7 @@ namespace fs {
 // (same layout as the context's own buffer); allocates nothing.
 int launch_elements_to(fs_ctx *c, int precision, void *ke)
 {
+    c->fx_marks.launch();
     if (c->mesh.nelem == 0) return FS_OK;
     return run_elements(c, precision, ke);
 }

@@ -26,4 +26,19 @@ uint64_t rows_reserve(Rows *r, uint64_t marks, uint64_t want, uint64_t group, ui
     return std::min<uint64_t>(want, fs::fx_groups_held(r->cap, marks, group));
 }
 
+// a sequence of events: l(aunch), m(ade), R(ead with the flag set), r(ead without);
+// the number of elements' redos
+int marks_events(const char *events)
+{
+    fs::FxMarks marks;
+    int redos = 0;
+    for (; *events; events++) {
+        if (*events == 'l') marks.launch();
+        if (*events == 'm') marks.made();
+        if (*events == 'R') redos += marks.redo(true);
+        if (*events == 'r') redos += marks.redo(false);
+    }
+    return redos;
+}
+
 }
