@@ -47,7 +47,8 @@ __device__ __forceinline__ void beam_load(const MeshDev &m, const BeamDev &b, in
     }
 }
 
-__device__ __forceinline__ void beam_prepare_rank(const MeshDev &m, const BeamDev &b, int64_t r, bool velocities,
+template <bool DIVIDE>
+__device__ __forceinline__ bool beam_prepare_rank(const MeshDev &m, const BeamDev &b, int64_t r, bool velocities,
                                                   int mass_type, BeamElem &e)
 {
     double x0[2][3], xt[2][3], R[2][3][3], v[2][6];
@@ -57,24 +58,19 @@ __device__ __forceinline__ void beam_prepare_rank(const MeshDev &m, const BeamDe
             const int node = m.conn[r * 2 + a];
             for (int k = 0; k < 6; k++) v[a][k] = b.v1 ? b.v1[(int64_t)k * m.nnodes + node] : 0.0;
         }
-    beam_prepare(x0, xt, R, velocities ? v : nullptr, b.sec[r], b.E, b.G, b.rho, mass_type, e);
+    return beam_prepare_by<DIVIDE>(x0, xt, R, velocities ? v : nullptr, b.sec[r], b.E, b.G, b.rho, mass_type, e);
 }
 
 // upper node blocks (0,0), (0,1), (1,1) of element matrix WHICH
-template <int WHICH>
-__global__ void __launch_bounds__(128) k_beam_elements(const MeshDev m, const BeamDev b, int mass_type, double *ke)
+template <int WHICH, bool ANY>
+__device__ __forceinline__ void beam_store_blocks(const MeshDev &m, const BeamElem &e, int64_t r, double *out)
 {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m.nelem) return;
-    BeamElem e;
-    beam_prepare_rank(m, b, r, WHICH == FS_BEAM_GYROSCOPIC, mass_type, e);
-    double *out = ke + r * 108;
 #pragma unroll
     for (int a = 0; a < 2; a++)
 #pragma unroll
         for (int bb = a; bb < 2; bb++) {
             double acc[6][6];
-            beam_block<WHICH>(e, a, bb, acc);
+            beam_block<WHICH, ANY>(e, a, bb, acc);
             if (a != bb && m.conn[2 * r] > m.conn[2 * r + 1]) {  // the lower node's dofs as rows
 #pragma unroll
                 for (int i = 0; i < 6; i++)
@@ -89,14 +85,33 @@ __global__ void __launch_bounds__(128) k_beam_elements(const MeshDev m, const Be
         }
 }
 
-// restoring force (WHICH 4) and distributed load (WHICH 5) per element
+// an element beyond the quotients' range (BmRange), out of line
 template <int WHICH>
-__global__ void __launch_bounds__(128) k_beam_vectors(const MeshDev m, const BeamDev b, double *fe)
+__device__ __noinline__ void beam_element_divided(const MeshDev *m, const BeamDev *b, int64_t r, int mass_type, double *out)
+{
+    BeamElem e;
+    beam_prepare_rank<true>(*m, *b, r, WHICH == FS_BEAM_GYROSCOPIC, mass_type, e);
+    beam_store_blocks<WHICH, true>(*m, e, r, out);
+}
+
+template <int WHICH>
+__global__ void __launch_bounds__(128) k_beam_elements(const __grid_constant__ MeshDev m, const __grid_constant__ BeamDev b,
+                                                       int mass_type, double *ke)
 {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= m.nelem) return;
     BeamElem e;
-    beam_prepare_rank(m, b, r, false, 0, e);
+    double *out = ke + r * 108;
+    if (beam_prepare_rank<false>(m, b, r, WHICH == FS_BEAM_GYROSCOPIC, mass_type, e))
+        beam_element_divided<WHICH>(&m, &b, r, mass_type, out);
+    else
+        beam_store_blocks<WHICH, false>(m, e, r, out);
+}
+
+// restoring force (WHICH 4) and distributed load (WHICH 5) per element
+template <int WHICH>
+__device__ __forceinline__ void beam_store_vector(const BeamDev &b, const BeamElem &e, int64_t r, double *fe)
+{
     double out[12];
     if (WHICH == 4)
         beam_restoring(e, out);
@@ -105,6 +120,24 @@ __global__ void __launch_bounds__(128) k_beam_vectors(const MeshDev m, const Bea
     double2 *o2 = reinterpret_cast<double2 *>(fe + r * 12);
 #pragma unroll
     for (int q = 0; q < 6; q++) o2[q] = make_double2(out[2 * q], out[2 * q + 1]);
+}
+template <int WHICH>
+__device__ __noinline__ void beam_vector_divided(const MeshDev *m, const BeamDev *b, int64_t r, double *fe)
+{
+    BeamElem e;
+    beam_prepare_rank<true>(*m, *b, r, false, 0, e);
+    beam_store_vector<WHICH>(*b, e, r, fe);
+}
+template <int WHICH>
+__global__ void __launch_bounds__(128) k_beam_vectors(const __grid_constant__ MeshDev m, const __grid_constant__ BeamDev b, double *fe)
+{
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= m.nelem) return;
+    BeamElem e;
+    if (beam_prepare_rank<false>(m, b, r, false, 0, e))
+        beam_vector_divided<WHICH>(&m, &b, r, fe);
+    else
+        beam_store_vector<WHICH>(b, e, r, fe);
 }
 
 // node sums of element vectors in ascending assembly rank

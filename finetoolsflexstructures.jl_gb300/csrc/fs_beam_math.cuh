@@ -12,6 +12,8 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
+#include <string.h>
 
 #ifndef FS_HD
 #if defined(__CUDACC__)
@@ -38,12 +40,48 @@ struct BeamFrame {
 
 // a / b with y the rounded reciprocal of b, as every component over one length:
 // the quotient with one residual correction (Markstein, IBM J. Res. Dev. 34
-// (1990) 111), which rounds as the division does
+// (1990) 111), which rounds as the division does while a (if not zero), b and the
+// quotient are well within the normal numbers
 FS_HD double bm_quotient(double a, double b, double y)
 {
     const double q = a * y;
     return fma(fma(-b, q, a), y, q);
 }
+template <bool DIVIDE> FS_HD double bm_over(double a, double b, double y) { return DIVIDE ? a / b : bm_quotient(a, b, y); }
+
+// |x| as the high word of its bits
+FS_HD uint32_t bm_magnitude(double x)
+{
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)__double2hiint(x) & 0x7fffffffu;
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return (uint32_t)(u >> 32) & 0x7fffffffu;
+#endif
+}
+// Whether an element suits the quotients by reciprocals: its lengths, which no
+// component exceeds, are between 2^-900 and 2^900 and its natural stiffnesses below
+// 2^900 (a component or stiffness below 2^-900 may be off by its last bit).  One that
+// does not (no length, an infinite or undefined section property) is prepared
+// with divisions, out of line.  Looked at once an element: a branch at each
+// quotient would keep them from overlapping (637,200 elements, stiffness: 0.91 ms an
+// assembly against 0.69).
+struct BmRange {
+    uint32_t lo = 0x7fffffffu, hi = 0;
+    FS_HD void length(double x)
+    {
+        const uint32_t u = bm_magnitude(x);
+        lo = u < lo ? u : lo;
+        hi = u > hi ? u : hi;
+    }
+    FS_HD void stiffness(double x)
+    {
+        const uint32_t u = bm_magnitude(x);
+        hi = u > hi ? u : hi;
+    }
+    FS_HD bool left() const { return lo < (1023u - 900u) << 20 || hi > (1023u + 900u) << 20; }
+};
 
 FS_HD double bm_norm3(const double v[3])
 {
@@ -52,12 +90,13 @@ FS_HD double bm_norm3(const double v[3])
 
 // axis 3 = axis 1 x v normalised, axis 2 = axis 3 x axis 1 (the explicit
 // skew products of src/FESetL2BeamModule.jl:112-125, src/FEMMCorotBeamModule.jl:161-180)
-FS_HD void bm_complete_frame(double F[3][3], const double v[3])
+template <bool DIVIDE> FS_HD void bm_complete_frame(double F[3][3], const double v[3], BmRange &g)
 {
     double e3[3] = {F[1][0] * v[2] - F[2][0] * v[1], F[2][0] * v[0] - F[0][0] * v[2],
                     F[0][0] * v[1] - F[1][0] * v[0]};
     const double n3 = bm_norm3(e3), y3 = 1.0 / n3;
-    for (int i = 0; i < 3; i++) F[i][2] = bm_quotient(e3[i], n3, y3);
+    g.length(n3);
+    for (int i = 0; i < 3; i++) F[i][2] = bm_over<DIVIDE>(e3[i], n3, y3);
     F[0][1] = F[1][2] * F[2][0] - F[2][2] * F[1][0];
     F[1][1] = F[2][2] * F[0][0] - F[0][2] * F[2][0];
     F[2][1] = F[0][2] * F[1][0] - F[1][2] * F[0][0];
@@ -66,15 +105,17 @@ FS_HD void bm_complete_frame(double F[3][3], const double v[3])
 // local_frame_and_def! (src/FEMMCorotBeamModule.jl:208-243): current frame,
 // lengths and natural deformations from the initial and current nodal
 // positions and the nodal rotation matrices RI, RJ.
+template <bool DIVIDE>
 FS_HD void beam_frame(const double x0[2][3], const double xt[2][3], const double x1x2[3],
-                                           const double RI[3][3], const double RJ[3][3], BeamFrame &f)
+                                           const double RI[3][3], const double RJ[3][3], BeamFrame &f, BmRange &g)
 {
     double F0[3][3], d[3];
     for (int c = 0; c < 3; c++) d[c] = x0[1][c] - x0[0][c];
     f.L0 = bm_norm3(d);
     const double y0 = 1.0 / f.L0;
-    for (int c = 0; c < 3; c++) F0[c][0] = bm_quotient(d[c], f.L0, y0);
-    bm_complete_frame(F0, x1x2);
+    g.length(f.L0);
+    for (int c = 0; c < 3; c++) F0[c][0] = bm_over<DIVIDE>(d[c], f.L0, y0);
+    bm_complete_frame<DIVIDE>(F0, x1x2, g);
     // nodal cross-section frames FtI = RI F0, FtJ = RJ F0
     double FI[3][3], FJ[3][3];
     for (int i = 0; i < 3; i++)
@@ -90,9 +131,10 @@ FS_HD void beam_frame(const double x0[2][3], const double xt[2][3], const double
     for (int c = 0; c < 3; c++) d[c] = xt[1][c] - xt[0][c];
     f.L1 = bm_norm3(d);
     f.y1 = 1.0 / f.L1;
-    for (int c = 0; c < 3; c++) f.Ft[c][0] = bm_quotient(d[c], f.L1, f.y1);
+    g.length(f.L1);
+    for (int c = 0; c < 3; c++) f.Ft[c][0] = bm_over<DIVIDE>(d[c], f.L1, f.y1);
     double v[3] = {FI[0][1] + FJ[0][1], FI[1][1] + FJ[1][1], FI[2][1] + FJ[2][1]};
-    bm_complete_frame(f.Ft, v);
+    bm_complete_frame<DIVIDE>(f.Ft, v, g);
     // components of the nodal frames in the element frame: L = Ft' F
     double LI[3][3], LJ[3][3];
     for (int i = 0; i < 3; i++)
@@ -118,14 +160,15 @@ FS_HD void beam_frame(const double x0[2][3], const double xt[2][3], const double
 // natural_stiffness! (src/FEMMCorotBeamModule.jl:729-779): diagonal DN,
 // Bernoulli when either shear area is infinite, else Timoshenko.
 // y = 1 / L.
+template <bool DIVIDE>
 FS_HD void beam_natural_stiffness(const BeamSection &s, double E, double G, double L, double y, double DN[6])
 {
-    DN[0] = bm_quotient(E * s.A, L, y);
-    DN[1] = bm_quotient(E * s.I3, L, y);
-    DN[3] = bm_quotient(E * s.I2, L, y);
-    DN[5] = bm_quotient(G * s.J, L, y);
-    DN[2] = bm_quotient(3 * E * s.I3, L, y);
-    DN[4] = bm_quotient(3 * E * s.I2, L, y);
+    DN[0] = bm_over<DIVIDE>(E * s.A, L, y);
+    DN[1] = bm_over<DIVIDE>(E * s.I3, L, y);
+    DN[3] = bm_over<DIVIDE>(E * s.I2, L, y);
+    DN[5] = bm_over<DIVIDE>(G * s.J, L, y);
+    DN[2] = bm_over<DIVIDE>(3 * E * s.I3, L, y);
+    DN[4] = bm_over<DIVIDE>(3 * E * s.I2, L, y);
     if (!(isinf(s.A2s) || isinf(s.A3s))) {
         const double Phi3 = 12 * E * s.I3 / (G * s.A2s * L * L);
         const double Phi2 = 12 * E * s.I2 / (G * s.A3s * L * L);
@@ -287,15 +330,19 @@ struct BeamElem {
 };
 
 // x0, xt: initial and current nodal positions; R: nodal rotation matrices;
-// v: nodal velocities (6 per node, gyroscopic only; null for none).
-FS_HD void beam_prepare(const double x0[2][3], const double xt[2][3], const double R[2][3][3], const double (*v)[6],
-                        const BeamSection &s, double E, double G, double rho, int mass_type, BeamElem &e)
+// v: nodal velocities (6 per node, gyroscopic only; null for none).  Returns whether
+// the element left the quotients' range (it is then to be prepared with DIVIDE).
+template <bool DIVIDE>
+FS_HD bool beam_prepare_by(const double x0[2][3], const double xt[2][3], const double R[2][3][3], const double (*v)[6],
+                           const BeamSection &s, double E, double G, double rho, int mass_type, BeamElem &e)
 {
+    BmRange g;
     e.s = s;
     e.rho = rho;
     e.mass_type = mass_type;
-    beam_frame(x0, xt, s.x1x2, R[0], R[1], e.f);
-    beam_natural_stiffness(s, E, G, e.f.L1, e.f.y1, e.DN);
+    beam_frame<DIVIDE>(x0, xt, s.x1x2, R[0], R[1], e.f, g);
+    beam_natural_stiffness<DIVIDE>(s, E, G, e.f.L1, e.f.y1, e.DN);
+    for (int k = 0; k < 6; k++) g.stiffness(e.DN[k]);
     for (int k = 0; k < 6; k++) e.PN[k] = e.DN[k] * e.f.dN[k];
     // angular velocity of the element frame from the nodal velocities
     // (gyroscopic, src/FEMMCorotBeamModule.jl:926-935)
@@ -313,13 +360,34 @@ FS_HD void beam_prepare(const double x0[2][3], const double xt[2][3], const doub
     e.OS[0][0] = 0.0;    e.OS[0][1] = -Om[2]; e.OS[0][2] = Om[1];
     e.OS[1][0] = Om[2];  e.OS[1][1] = 0.0;    e.OS[1][2] = -Om[0];
     e.OS[2][0] = -Om[1]; e.OS[2][1] = Om[0];  e.OS[2][2] = 0.0;
+    return !DIVIDE && g.left();
+}
+FS_HD void beam_prepare(const double x0[2][3], const double xt[2][3], const double R[2][3][3], const double (*v)[6],
+                        const BeamSection &s, double E, double G, double rho, int mass_type, BeamElem &e)
+{
+    if (beam_prepare_by<false>(x0, xt, R, v, s, E, G, rho, mass_type, e))
+        beam_prepare_by<true>(x0, xt, R, v, s, E, G, rho, mass_type, e);
 }
 
 // Node block (a, b) of the global element matrix WHICH (0 stiffness,
-// 1 geometric stiffness, 2 mass, 3 gyroscopic): acc[i][j] = K[6a+i][6b+j].
-template <int WHICH>
+// 1 geometric stiffness, 2 mass, 3 gyroscopic): acc[i][j] = K[6a+i][6b+j].  ANY: the
+// element may have an infinite or undefined DN_k.
+template <int WHICH, bool ANY>
 FS_HD void beam_block_raw(const BeamElem &e, int a, int b, double acc[6][6])
 {
+    bool all = false;
+    if (WHICH == 0 && ANY)
+        for (int k = 0; k < 6; k++) all = all || bm_magnitude(e.DN[k]) >= 0x7ff00000u;
+    if (all) {
+        // a zero times an infinity is undefined: every term counts
+        for (int i = 0; i < 36; i++) acc[i / 6][i % 6] = 0.0;
+        for (int k = 0; k < 6; k++) {
+            double g[12];
+            beam_row(k, e.f.Ft, e.f.L1, g);
+            for (int i = 0; i < 36; i++) acc[i / 6][i % 6] += e.DN[k] * g[6 * a + i / 6] * g[6 * b + i % 6];
+        }
+        return;
+    }
     if (WHICH == 0) {
         // K = sum_k DN_k g_k g_k' with, f_c the columns of Ft and h = 2 / L,
         // g_0 = (-f0, 0, f0, 0), g_1 = (0, f2, 0, -f2), g_2 = (h f1, f2, -h f1, f2),
@@ -379,10 +447,10 @@ FS_HD void beam_block_raw(const BeamElem &e, int a, int b, double acc[6][6])
 // Node block (a, b); a diagonal block is made exactly symmetric from its
 // upper triangle (as complete_lt! does), so the assembled matrix is symmetric
 // to the bit.
-template <int WHICH>
+template <int WHICH, bool ANY = true>
 FS_HD void beam_block(const BeamElem &e, int a, int b, double acc[6][6])
 {
-    beam_block_raw<WHICH>(e, a, b, acc);
+    beam_block_raw<WHICH, ANY>(e, a, b, acc);
     if (a == b)
         for (int i = 0; i < 6; i++)
             for (int j = i + 1; j < 6; j++) acc[j][i] = acc[i][j];
