@@ -852,10 +852,7 @@ int fs_explicit_setup(fs_ctx *c, int precision, const double *invMC, const doubl
         return set_err(c, FS_ERR_BAD_INPUT, "unknown precision");
     if (!(dt > 0.0)) return set_err(c, FS_ERR_BAD_INPUT, "time step must be positive");
     auto &x = c->ex;
-    if (x.exec) cudaGraphExecDestroy(x.exec);
-    if (x.graph) cudaGraphDestroy(x.graph);
-    x.exec = nullptr;
-    x.graph = nullptr;
+    end_explicit(c);  // no state until all buffers are there: an allocation may fail
     x.load = false;
     int64_t n = c->mat_n;
     x.n = n;
