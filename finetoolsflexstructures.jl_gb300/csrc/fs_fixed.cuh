@@ -7,12 +7,19 @@
 //
 // A number is X 2^(E-58), X an integer of about 58 bits and sign, E an exponent
 // shared by a group of numbers and above the largest of them: it is kept to
-// 2^-58 of the group's largest, a quarter of a per cent of that one's last
-// double bit.  X is split in two limbs, X = h 2^29 + l with |l| <= 2^28; a
-// product keeps h h' (into one 64-bit sum) and h l' + l h' (into another), three
-// multiply-adds, and drops l l' (below 2^-60 of the largest product).  Both sums
-// are exact for up to 12 products of numbers up to 1.41 times their group's
-// largest.  A sum becomes an X again by one rounding, a double by another.
+// 2^-58 of the group's largest, whose last bit in double is 2^-53 of it.  Numbers
+// below 2^-5 of the largest thus keep fewer bits than in double; the groups are
+// chosen so that this does not matter to their products (fs_elem_fixed.cuh).  X is
+// split in two limbs, X = h 2^29 + l with |l| <= 2^28; a product keeps h h' (into
+// one 64-bit sum) and h l' + l h' (into another), three multiply-adds, and drops
+// l l' (below 2^-60 of the largest product).  A sum becomes an X again by one
+// rounding, a double by another.
+//
+// The sums are exact while they fit 63 bits: products of X up to c 2^58 and c' 2^58
+// may be up to 32 / (c c') of them.  Entries and products (triangle; quadrilateral,
+// whose groups M, R and of layered dofs have a bit to spare): M below 2 and 3, 1 and
+// 12; T 1.2 and 5, 20; R 1.42 and 5, 0.71 and 20; T R 8.6 and 17.1 in sum; layered
+// 1 and 13, 0.5 and 33.  Largest: T of a quadrilateral, 28.8 of 32.
 //
 // Group exponents are far from a double's limits and all numbers finite: the
 // kernels check this (fx_usable) and take their double path otherwise.
