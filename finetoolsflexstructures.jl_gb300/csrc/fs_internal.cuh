@@ -52,7 +52,7 @@ __host__ __device__ __forceinline__ int stored_entry(int a, int b, int nen, cons
     return (a <= b ? ub(a, b, nen) : ub(b, a, nen)) * 36 + (rows_a ? 6 * i + j : 6 * j + i);
 }
 static const int GATHER_GROUP = 64;         // nodes whose own blocks lie together in the gather's list
-static const int MAX_NBRS = 255;            // neighbour nodes of one node (slots are 8-bit)
+static const int MAX_NBRS = 255;            // neighbour nodes of one node (of 64 elements with 4 nodes, 193 at most)
 
 struct MeshDev {
     int etype = -1, nen = 0;

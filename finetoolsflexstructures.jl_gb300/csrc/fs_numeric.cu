@@ -332,8 +332,8 @@ int launch_elements_to(fs_ctx *c, int precision, void *ke)
 // tile-shape autotuner
 // ---------------------------------------------------------------------------
 // Candidates: elements per block of the element kernel (T3: 32, 64, 128;
-// Q4: 8, 16, 32, as far as their shared memory fits in 227 KB) and the block
-// size of the gather (4, 8, 16 times 36 threads).  Each candidate is timed on the
+// Q4: 8, 16, 32, as far as their shared memory fits in 227 KB) and the warps of
+// a block of the gather (4, 8, 16; five node-block pairs each).  Each candidate is timed on the
 // context's own mesh with CUDA events (best of three launches), the element
 // kernel first, then the gather on its output.  The choice is keyed on
 // element family, precision, the average-K option, whether exact zeros are

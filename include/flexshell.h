@@ -46,7 +46,12 @@ extern "C" {
 #define FS_COROTBEAM 4  /* FEMMCorotBeam (2-node L2 beams), src/FEMMCorotBeamModule.jl */
 
 /* arithmetic of the element strain rows and Gram products */
-#define FS_FP64 0       /* double precision: the drop-in                     */
+#define FS_FP64 0       /* double precision: the drop-in.  T3FF (average B), Q4RS
+                           and the layered elements form part of it in 58-bit
+                           fixed point, no less exactly than in double; with
+                           FS_ASM_SPARSE_SYMM, which drops exact zeros, all is
+                           double, so the two assemblers' entries may differ in
+                           the last bits                                       */
 #define FS_MIXED 1      /* float element arithmetic on element frames and
                            coordinates formed in double (the Q4 Gauss-point
                            frames and drilling factor in float); CSR values
@@ -185,8 +190,9 @@ int fs_timings(const fs_ctx *ctx, double *out, int n);
 /* Tile-shape autotuner of the shell assembly (elements per block of the
  * element kernel; warps per block of the CSR gather).  Mode 1 (the default;
  * environment FLEXSHELL_AUTOTUNE=0 makes 0 the default): the first fs_stiffness
- * call for a new key (element family, precision, average-K option, log2 of the
- * element count; meshes of at least 4096 elements) times every candidate on the
+ * call for a new key (element family, precision, average-K option, whether
+ * exact zeros are dropped, log2 of the element count; meshes of at least 4096
+ * elements) times every candidate on the
  * context's mesh and the choice is reused by the whole process; 0: built-in
  * shapes; 2: re-tune on the next call; 3: built-in shapes
  * with every pair summed by both nodes.  No choice changes the results. */
