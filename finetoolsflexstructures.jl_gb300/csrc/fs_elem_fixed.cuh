@@ -734,6 +734,7 @@ template <int NP, int BS, int BSS, bool DIAG, class X>
 FS_HD void fx_block_bottom(FxSlots rows, int step, int p, int q, FxSlots drill, const X &ex, double o[3][6])
 {
     const FxNode a = ex.node(p), b = ex.node(q);
+    const int top = 2 * (a.q > ex.r ? a.q : ex.r);  // the larger of the rows' and the drilling row's products
     FxSums rt, rr, dd;
     rt.zero();
     rr.zero();
@@ -762,8 +763,11 @@ FS_HD void fx_block_bottom(FxSlots rows, int step, int p, int q, FxSlots drill, 
         }
         FS_UNROLL
         for (int j = DIAG ? i : 0; j < 3; j++) {
-            o[i][3 + j] = rr.value(i, j, a.q + b.q);
-            if (DIAG) o[i][3 + j] += dd.value(i, j, 2 * ex.r);
+            if (DIAG)
+                o[i][3 + j] = fx_double(FxSum{fx_shift(fx_round(FxSum{rr.hh[i][j], rr.c[i][j]}), top - 2 * a.q) +
+                                                  fx_shift(fx_round(FxSum{dd.hh[i][j], dd.c[i][j]}), top - 2 * ex.r), 0}, top);
+            else
+                o[i][3 + j] = rr.value(i, j, a.q + b.q);
             if (DIAG && j > i) o[j][3 + i] = o[i][3 + j];
         }
     }
