@@ -17,7 +17,7 @@
 // unrolled, since the compiler copies every 64-bit sum of a rolled loop.  In one
 // kernel the two need the first one's registers and shared memory for the rows,
 // 1 KB a T3 element, which leaves 5 warps an SM: 4.4 ms against 3.5 ms (T3,
-// 1024 x 1024) and 4.2 against 3.2 ms (Q4, 512 x 512); all in double 8.0 and
+// 1024 x 1024) and 4.2 against 3.3 ms (Q4, 512 x 512); all in double 8.0 and
 // 7.5 ms.
 //
 // A chunk's rows pass through a buffer of at most 1 GiB.  Small chunks would
